@@ -30,7 +30,7 @@
 // window is (h >> 5) + (w >> 5) and its bit shift is h & 31 for every lane.
 //
 // Buckets of at most 32 keys (nearly all of them) keep one key per lane in
-// registers and test collisions with __match_any_sync; for at most 8 keys the
+// registers and test collisions when they mark; for at most 8 keys the
 // offset search also keeps every slot in registers (as 4 or 8 slots, the unused
 // ones repeating slot 0), for 9..32 keys it reads them from shared memory four at
 // a time.  Larger buckets read their keys from the
@@ -308,10 +308,45 @@ __device__ __forceinline__ void mark_if(uint32_t *occ, uint32_t q, uint32_t ps, 
         : "memory");
 }
 
+// Two keys of a bucket on one slot reject the pilot counter (search.comp:44-70).  That is
+// rare (1 % of the tries of buckets of at most 32 keys at lambda 7), so it is tested only once
+// a free offset is found, with the shared-memory atomics that the marks need anyway: two lanes
+// on one slot show as a bit that was set already.  __match_any_sync on every try, as before,
+// takes 354-378 cycles and occupies an SM's unit for 59-64 cycles per warp (measured alone on a
+// B200; atomicOr with its result: 42 and 1.6).  At 10^8 u64 keys (lambda 7, P 2500) the search
+// took 7.65 ms with it and 7.17 ms without.
+
+// Marks slot q (and its mirror) of every lane that is `on`, or marks nothing and returns
+// false when two of the lanes hold the same slot.  The slots were free before.
+__device__ __forceinline__ bool mark_distinct(uint32_t *occ, uint32_t q, uint32_t ps, bool on) {
+    const uint32_t bit = 1u << (q & 31);
+    const uint32_t old = on ? atomicOr(&occ[q >> 5], bit) : 0u;
+    if (__any_sync(kFullMask, on && (old & bit))) {
+        if (on) atomicAnd(&occ[q >> 5], ~bit);
+        __syncwarp();
+        return false;
+    }
+    const uint32_t m = q + ps;
+    if (on) atomicOr(&occ[m >> 5], 1u << (m & 31));
+    __syncwarp();
+    return true;
+}
+
+// Whether the slots of the lanes that are `on` are distinct, tested in the warp's own clear
+// collision scratch (left clear): for searches that do not mark.
+__device__ __forceinline__ bool slots_distinct(uint32_t *scr, uint32_t q, bool on) {
+    const uint32_t bit = 1u << (q & 31);
+    const uint32_t old = on ? atomicOr(&scr[q >> 5], bit) : 0u;
+    const bool hit = __any_sync(kFullMask, on && (old & bit));
+    if (on) scr[q >> 5] = 0;
+    __syncwarp();
+    return !hit;
+}
+
 // A bucket of at most S keys (S = 4 or 8) in a partition of at most 3072 slots: the warp
 // hashes 32 / S pilot counters at once (lane t * S + i holds key i under counter k0 + t; lanes
 // past the bucket hold key 0, the padding the scan expects) and tests them in counter order, so
-// a counter that fails costs no new hash or collision test.  Same result as trying
+// a counter that fails costs no new hash.  Same result as trying
 // k = 0, 1, 2, ... one at a time (search.comp:105-124).  With MARK the slots are marked and
 // *pilot written; without, nothing is marked and the bucket pipeline gets the counter, the
 // offset and (lanes < s) the lane's slot in *k_out, *o_out, *q_out.
@@ -321,7 +356,6 @@ __device__ __forceinline__ uint32_t place_batched(const WarpSmem &ws, uint2 L, u
                                                   uint32_t *k_out = nullptr, uint32_t *o_out = nullptr,
                                                   uint32_t *q_out = nullptr) {
     constexpr int G = 32 / S;
-    constexpr uint32_t kGroupMask = (1u << S) - 1u;
     const int t = lane / S, i = lane % S;
     const bool key = i < (int)s;
     const uint32_t lx = __shfl_sync(kFullMask, L.x, key ? i : 0), ly = __shfl_sync(kFullMask, L.y, key ? i : 0);
@@ -329,30 +363,22 @@ __device__ __forceinline__ uint32_t place_batched(const WarpSmem &ws, uint2 L, u
     const bool mine = lane < (int)s;
     for (uint32_t k0 = 0;; k0 += G) {
         const uint32_t hk = fm.mod(pilot_hash(lx, ly, k0 + (uint32_t)t));
-        // Two keys of one counter on one slot: the counter rides above the slot (slots < 2^16).
-        uint32_t coll = 0;
-        if (s > 1) {
-            const uint32_t v = key ? (hk | ((uint32_t)t << 24)) : (0x80000000u | (uint32_t)lane);
-            const uint32_t m = __match_any_sync(kFullMask, v);
-            coll = __ballot_sync(kFullMask, key && (m & (m - 1)) != 0);
-        }
         const uint32_t pk = pack_slot(hk);
 #pragma unroll 1
         for (int u = 0; u < G; u++) {
             const uint32_t k = k0 + (uint32_t)u;
             if (k >= k_lim) return PHOBIC_ERR_SEARCH_LIMIT;
             if (k == kDupCheckAt && s > 1 && has_duplicate_key(L, s, lane)) return PHOBIC_ERR_DUPLICATE_KEY;
-            if ((coll >> (u * S)) & kGroupMask) continue;
             const uint32_t hp = __shfl_sync(kFullMask, pk, u * S + pick);
             const uint32_t o = first_free_offset_unr<S>(ws.occ, hp, ps, rounds, lane, ws.occ_lo, ws.occ_hi);
             if (o == kNone) continue;
             uint32_t q = __shfl_sync(kFullMask, hk, u * S + pick) + o;
             q = q >= ps ? q - ps : q;
             if constexpr (MARK) {
-                mark_if(ws.occ, q, ps, mine && PHB_CHECK(!mine || q < ps));
-                __syncwarp();
+                if (!mark_distinct(ws.occ, q, ps, mine && PHB_CHECK(!mine || q < ps))) continue;
                 *pilot = o + ps * k;
             } else {
+                if (!slots_distinct(ws.scr, q, mine && PHB_CHECK(!mine || q < ps))) continue;
                 *k_out = k;
                 *o_out = o;
                 *q_out = q;
@@ -367,20 +393,14 @@ __device__ __forceinline__ uint32_t place_small(const WarpSmem &ws, uint2 L, uin
                                                 uint32_t k_lim, uint32_t rounds, int lane, uint32_t *pilot) {
     const bool mine = lane < (int)s;
     const uint32_t padded = (s + 3) & ~3u;
-    // Every lane hashes (no divergent branch); lanes past the bucket take distinct
-    // out-of-range values, so they never collide.  The hash of counter k + 1 is formed
+    // Every lane hashes (no divergent branch).  The hash of counter k + 1 is formed
     // while counter k is tested: the two dependency chains overlap.
     uint32_t hk_next = fm.mod(pilot_hash(L.x, L.y, 0u));
     for (uint32_t k = 0; k < k_lim; k++) {
         if (k == kDupCheckAt && s > 1 && has_duplicate_key(L, s, lane)) return PHOBIC_ERR_DUPLICATE_KEY;
         const uint32_t hk = hk_next;
         hk_next = fm.mod(pilot_hash(L.x, L.y, k + 1));
-        const uint32_t h = mine ? hk : (0x80000000u | lane);
-        if (s > 1) {
-            uint32_t m = __match_any_sync(kFullMask, h);
-            if (__any_sync(kFullMask, mine && (m & (m - 1)) != 0)) continue;
-        }
-        const uint32_t hp = pack_slot(__shfl_sync(kFullMask, h, mine ? lane : 0));
+        const uint32_t hp = pack_slot(__shfl_sync(kFullMask, hk, mine ? lane : 0));
         uint32_t o;  // buckets of at most 8 keys with at most three rounds go to place_batched
         if (s <= 4) o = first_free_offset_reg<4>(ws.occ, hp, ps, lane, ws.occ_lo, ws.occ_hi);
         else if (s <= 8) o = first_free_offset_reg<8>(ws.occ, hp, ps, lane, ws.occ_lo, ws.occ_hi);
@@ -393,8 +413,7 @@ __device__ __forceinline__ uint32_t place_small(const WarpSmem &ws, uint2 L, uin
         if (o == kNone) continue;
         uint32_t q = hk + o;
         q = q >= ps ? q - ps : q;
-        mark_if(ws.occ, q, ps, mine && PHB_CHECK(!mine || q < ps));
-        __syncwarp();
+        if (!mark_distinct(ws.occ, q, ps, mine && PHB_CHECK(!mine || q < ps))) continue;
         *pilot = o + ps * k;
         return PHOBIC_OK;
     }
@@ -544,6 +563,20 @@ __device__ __forceinline__ void discard_partition_copy(const uint2 *so, uint32_t
         asm volatile("discard.global.L2 [%0], 128;" ::"l"(x) : "memory");
 }
 
+// Lanes holding the same BITS-bit value: one vote per bit, all in flight together (nine votes
+// take an SM about 15 cycles, __match_any_sync 60).
+template <int BITS>
+__device__ __forceinline__ uint32_t same_value_lanes(uint32_t v) {
+    uint32_t same = kFullMask;
+#pragma unroll
+    for (int b = 0; b < BITS; b++) {
+        const bool on = (v >> b) & 1u;
+        const uint32_t set = __ballot_sync(kFullMask, on);
+        same &= on ? set : ~set;
+    }
+    return same;
+}
+
 // Preparation of one partition by one warp: bucket histogram, search order (in
 // ws.sched), bucket-ordered keys (in a.sorted), pilot 0 for empty buckets, a clear
 // bitmap and collision scratch.  *nonempty = buckets to search; *skip = true when the
@@ -625,7 +658,7 @@ __device__ __forceinline__ uint32_t prep_partition(const SearchArgs &a, const Wa
     for (uint32_t c0 = 0; c0 < B; c0 += 32) {
         const int bi = (int)B - 1 - (int)(c0 + lane);
         const uint32_t s = bi >= 0 ? half_get(ws.cnt32, bi) : 0u;
-        const uint32_t peers = __match_any_sync(kFullMask, s ? s : 0x10000u + lane);
+        const uint32_t peers = same_value_lanes<9>(s);
         const uint32_t r = __popc(peers & lanemask_lt());
         const uint32_t bin = kBins - s;
         if (s) {
@@ -748,12 +781,7 @@ __device__ __forceinline__ uint32_t try_small(const WarpSmem &ws, uint32_t s, ui
                                               uint32_t rounds, int lane, uint32_t *o_out) {
     const bool mine = lane < (int)s;
     const uint32_t padded = (s + 3) & ~3u;
-    const uint32_t h = mine ? hk : (0x80000000u | lane);
-    if (s > 1) {
-        uint32_t m = __match_any_sync(kFullMask, h);
-        if (__any_sync(kFullMask, mine && (m & (m - 1)) != 0)) return kTryNone;
-    }
-    const uint32_t hp = pack_slot(__shfl_sync(kFullMask, h, mine ? lane : 0));
+    const uint32_t hp = pack_slot(__shfl_sync(kFullMask, hk, mine ? lane : 0));
     uint32_t o;
     if (s <= 8 && rounds <= 3) {
         if (s <= 4) o = first_free_offset_unr<4>(ws.occ, hp, ps, rounds, lane, ws.occ_lo, ws.occ_hi);
@@ -766,7 +794,7 @@ __device__ __forceinline__ uint32_t try_small(const WarpSmem &ws, uint32_t s, ui
         o = first_free_offset(ws.occ, ws.hs, s, ps, lane, ws.occ_lo, ws.occ_hi);
         __syncwarp();
     }
-    if (o == kNone) return kTryNone;
+    if (o == kNone || !slots_distinct(ws.scr, hk, mine && PHB_CHECK(!mine || hk < ps))) return kTryNone;
     *o_out = o;
     return kTryFound;
 }
