@@ -94,8 +94,8 @@ typedef struct phobic_timings {
     float input_transfer;     /* host -> device copy of the keys (overlapped with bucket_sizes) */
     float bucket_sizes;       /* hash + partition count (kernel K1) */
     float partition_offsets;  /* decoupled-lookback scan (kernel K2) */
-    float key_redistribution; /* partition scatter (kernel K3) */
-    float search;             /* bucket sort + pilot search (kernel K4) */
+    float key_redistribution; /* partition scatter + bucket sort (kernels K3) */
+    float search;             /* pilot search (kernel K4) */
     float result_transfer;    /* device -> host copy of pilots and offsets */
     float total;              /* first event to last event */
     uint32_t kernels;         /* kernels launched by the call */

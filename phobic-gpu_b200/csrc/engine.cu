@@ -4,11 +4,11 @@
 //   reference stage (mphf_builder.h)           here
 //   initialHash (host, :201-216)          ->  K1 map_count (XXH3 on the device)
 //   input_transfer (:233-238)             ->  H2D of the raw keys (no 16-byte Key array)
-//   bucket_sizes (:153-159)               ->  K1 (partition counts) + K4 (bucket counts)
-//   bucket_sorting (:162-167)             ->  K4 (shared memory, per partition)
+//   bucket_sizes (:153-159)               ->  K1 (partition counts) + K3c (bucket counts)
+//   bucket_sorting (:162-167)             ->  K3c (shared memory, per partition)
 //   partition_offsets (:169-174)          ->  K2 decoupled-lookback scan
 //   apply_partition_offsets (:176-180)    ->  K2 cursors + K3
-//   key_redistribution (:182-187)         ->  K3 + K4
+//   key_redistribution (:182-187)         ->  K3 + K3c
 //   search (:189-194)                     ->  K4
 //   result_transfer (:196-261)            ->  D2H of pilots and offsets
 //
@@ -380,7 +380,7 @@ phobic_status check_params(const phobic_params *params, uint32_t *cap, uint32_t 
     *cap = params->max_partition_size ? params->max_partition_size : default_max_partition(params->partition_size);
     *k_max = params->max_pilot_counter ? params->max_pilot_counter : kDefaultMaxPilot;
     if (*cap > 65535) return bad("max_partition_size must be <= 65535");
-    if (search_warps_per_cta(params->buckets, *cap) < 1)
+    if (!search_accepts(params->buckets, *cap))
         return bad("buckets/partition capacity exceed the search kernel's shared memory");
     return PHOBIC_OK;
 }
@@ -574,10 +574,10 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
     MapArgs ma{d_desc, d_kb, nsets, B, N, d_fulcs, d_count, d_mapped, d_dbg_keys, d_lowers, d_bkt, d_err,
                (uint32_t)M, plan.stride, plan.chunk};
     ScanArgs sa{d_count, d_G, nullptr, (uint32_t)MS, d_tiles, reinterpret_cast<uint32_t *>(d_tiles + tiles), nsets,
-                d_err, 0};
+                d_err, 0, d_pcur, d_bincur, plan.stride, wshift};
     PartArgs pa{d_inter, d_bincur, d_pcur, wshift, (uint32_t)((M + (1ull << wshift) - 1) >> wshift), (uint32_t)M};
     SearchArgs qa{d_desc, d_pb, nsets, (uint32_t)M, d_G, plan.stride, d_lowers, d_bkt, d_sorted, d_dbg_sizes, B, cap,
-                  k_max, d_queue, d_err, d_pcur};
+                  k_max, d_queue, d_err, d_pcur, P};
 
     // The device stages, from the per-build memsets to the status copy: enqueued one by one,
     // or under stream capture (the stage events then become event-record nodes of the graph).
@@ -591,7 +591,7 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
         PHB_TRY(cudaMemsetAsync(d_tiles, 0, 8 * (size_t)tiles + 8, s), "memset");
         if (M == 0) PHB_TRY(cudaMemsetAsync(d_G, 0, 4, s), "memset");
         PHB_TRY(record(w.ev[1]), "event");
-        // K1, scan, size check, two partition passes, search; none when there are no keys.
+        // K1, scan, two partition passes, bucket order, search; none when there are no keys.
         {
             StageRange r("bucket_sizes (K1)");
             PHB_TRY(launch_map_count(kind, ma, plan, s), "K1 map_count");
@@ -603,11 +603,11 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
             StageRange r("partition_offsets (K2)");
             PHB_TRY(launch_scan(sa, s), "K2 scan");
         }
-        PHB_TRY(launch_check_sizes(d_G, (uint32_t)M, plan.stride, cap, d_pb, nsets, d_err, &pa, s), "K2 size check");
         PHB_TRY(record(w.ev[3]), "event");
         {
             StageRange r("key_redistribution (K3)");
             PHB_TRY(launch_partition(kind, ma, pa, w.sm_count, s), "K3 partition");
+            PHB_TRY(launch_order(qa, w.sm_count, s), "K3 order");
         }
         PHB_TRY(record(w.ev[4]), "event");
         {

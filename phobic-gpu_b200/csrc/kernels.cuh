@@ -2,9 +2,9 @@
 //
 //   K1 map_count  keys -> key counts per (partition, chunk)         (kernels_map.cu)
 //   K2 scan       counts -> record offsets (= scatter cursors)      (kernels_scan.cu)
-//                 + partition size check
 //   K3 scatter    keys -> partition-contiguous (lower pair, bucket) records
-//   K4 search     per partition: bucket sort + pilot search         (kernels_search.cu)
+//   K3c order     per partition: size check, bucket sort            (kernels_order.cu)
+//   K4 search     per partition: pilot search                       (kernels_search.cu)
 //   Q  query      keys -> slots, bijection check                    (kernels_query.cu)
 //
 // Every kernel works on a list of key sets.  The partitions of all sets form one
@@ -121,6 +121,10 @@ struct ScanArgs {
     uint32_t nsets;
     unsigned long long *err;         // [nsets]
     unsigned long long wait_ns;      // bound of the look-back wait on a predecessor tile
+    // Two-pass partition (or null): offset of every partition (entry g * stride) and of every
+    // coarse bin's first partition.
+    uint32_t *pcur = nullptr, *bincur = nullptr;
+    uint32_t stride = 1, wshift = 0;
 };
 
 struct SearchArgs {
@@ -130,19 +134,24 @@ struct SearchArgs {
     uint32_t M;                 // global partitions
     const uint32_t *G;          // [M * gstride + 1] record offsets; partition g spans [G[g*gstride], G[(g+1)*gstride])
     uint32_t gstride;
-    const uint2 *lowers;        // partition-contiguous records
+    // Partition-contiguous records; K3c leaves a partition's search schedule in the place of its
+    // lower pairs (words 2 * G[g * gstride] ...).
+    const uint2 *lowers;
     const uint16_t *bkt;
-    uint2 *sorted;              // scratch, same indexing as lowers
+    uint2 *sorted;              // lower pairs in search order, same indexing as lowers
     uint32_t *debug_sizes;      // [M * buckets] or null
     uint32_t buckets;
     uint32_t cap;
     uint32_t k_max;
     uint32_t *queue;            // zeroed job counter
     unsigned long long *err;    // [nsets]
-    // [M] placement cursors after K3 (or null): partition g must end at its scanned offset,
-    // else its keys differed between K1 and K3.
-    const uint32_t *placed = nullptr;
+    // [M] placement cursors after K3: partition g must end at its scanned offset, else its keys
+    // differed between K1 and K3.  K3c replaces them by the number of nonempty buckets, or
+    // kPartSkipped | the status that the search reports (0 = reported before).
+    uint32_t *part_state;
+    uint32_t partition_size;    // P: expected keys per partition
 };
+constexpr uint32_t kPartSkipped = 0x80000000u;
 
 struct QueryArgs {
     uint32_t partitions;
@@ -177,18 +186,16 @@ __device__ __forceinline__ Key4 load_key(const void *data, const uint64_t *offse
 
 // Shared-memory bytes one warp of K4 needs for a partition capacity and bucket count.
 size_t search_warp_smem(uint32_t buckets, uint32_t cap);
+// Whether the build takes these parameters (they bound the shared memory of K3c and K4).
+bool search_accepts(uint32_t buckets, uint32_t cap);
+// K3c: size check, bucket sizes, search order and bucket-ordered keys of every partition.
+cudaError_t launch_order(const SearchArgs &a, int sm_count, cudaStream_t st);
 // Warps (= partitions in flight) per K4 CTA; 0 when one warp's state does not fit.
 int search_warps_per_cta(uint32_t buckets, uint32_t cap);
 
 cudaError_t launch_map_count(int kind, const MapArgs &a, const MapPlan &plan, cudaStream_t st);
 cudaError_t launch_scatter(int kind, const MapArgs &a, const MapPlan &plan, cudaStream_t st);
 cudaError_t launch_scan(const ScanArgs &a, cudaStream_t st);
-// Partition sizes out[(g+1)*stride] - out[g*stride] checked against cap (the search
-// bitmap capacity); an oversized partition is reported as PHOBIC_ERR_PARTITION_OVERFLOW.
-// With a PartArgs (else null) it also seeds the partition and bin cursors.
-cudaError_t launch_check_sizes(const uint32_t *out, uint32_t M, uint32_t stride, uint32_t cap,
-                               const uint32_t *part_base, uint32_t nsets, unsigned long long *err,
-                               const PartArgs *part, cudaStream_t st);
 // K3, two passes (pass 1 hashes the keys again, or reads K1's mapped records for strings).
 cudaError_t launch_partition(int kind, const MapArgs &a, const PartArgs &p, int sm_count, cudaStream_t st);
 // The scan with its first `skip` tile ids never handed out, so the tiles after them
@@ -214,6 +221,7 @@ size_t search_group_smem(uint32_t buckets, uint32_t cap, int W);
 // none; always 0 in the normal build); reset clears it.
 unsigned int check_line_map(bool reset);
 unsigned int check_line_part(bool reset);
+unsigned int check_line_order(bool reset);
 unsigned int check_line_search(bool reset);
 // splitmix64 stream on the device: out[i] = the finalizer of seed + (i + 1) * 0x9E3779B97F4A7C15
 // (synthetic keys of the autotuner).

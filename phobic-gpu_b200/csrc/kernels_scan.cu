@@ -6,8 +6,8 @@
 // (include/phobicGpu/mphf_builder.h:254-257): out[0] = 0, out[p + 1] = out[p] + size[p].
 // The scanned array is the (partition, chunk) count matrix of K1, so the prefix
 // is at once every partition's record offset and every chunk's scatter cursor.
-// A second small kernel checks every partition against the search bitmap
-// capacity, which the reference leaves unchecked (search.comp:21).
+// The tile that holds a partition's first entry also seeds its placement cursor and, for a
+// coarse bin's first partition, the bin's.
 //
 // Each CTA takes the next tile id from a counter, so every tile it waits on was
 // started before it; the wait on a predecessor is still bounded in time
@@ -92,12 +92,21 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(ScanArgs a) {
     __syncthreads();
 
     uint32_t run = s_prefix + s_warp[warp] + incl - sum;
+    // The next partition that starts at or after this thread's first entry.
+    const uint32_t b32 = (uint32_t)base;  // entries number less than 2^32
+    uint64_t g = a.pcur && base < a.m ? b32 / a.stride + (b32 % a.stride != 0) : 0, first = g * a.stride;
 #pragma unroll
     for (int j = 0; j < kScanItems; j++) {
         uint64_t idx = base + j;
         if (idx < a.m) {
             a.out[idx] = run;
             if (a.cursor) a.cursor[idx] = run;
+            if (a.pcur && idx == first) {
+                a.pcur[g] = run;
+                if ((g & ((1ull << a.wshift) - 1)) == 0) a.bincur[g >> a.wshift] = run;
+                g++;
+                first += a.stride;
+            }
         }
         run += v[j];
     }
@@ -111,32 +120,6 @@ cudaError_t launch_scan(const ScanArgs &a, cudaStream_t st) {
     ScanArgs b = a;
     if (!b.wait_ns) b.wait_ns = kSpinTimeoutNs;
     k_scan<<<tiles, kScanThreads, 0, st>>>(b);
-    return cudaGetLastError();
-}
-
-__global__ void k_check_sizes(const uint32_t *out, uint32_t M, uint32_t stride, uint32_t cap, const uint32_t *part_base,
-                              uint32_t nsets, unsigned long long *err, PartArgs part, bool seed) {
-    const uint32_t g = blockIdx.x * blockDim.x + threadIdx.x;
-    if (g >= M) return;
-    const uint32_t start = out[(size_t)g * stride];
-    if (seed) {
-        part.pcur[g] = start;
-        if ((g & ((1u << part.wshift) - 1)) == 0) part.bincur[g >> part.wshift] = start;
-    }
-    const uint32_t size = out[(size_t)(g + 1) * stride] - start;
-    if (size > cap) {
-        const uint32_t set = nsets == 1 ? 0u : find_set(part_base, nsets, g);
-        report_error(&err[set], g - part_base[set], PHOBIC_ERR_PARTITION_OVERFLOW);
-    }
-}
-
-cudaError_t launch_check_sizes(const uint32_t *out, uint32_t M, uint32_t stride, uint32_t cap,
-                               const uint32_t *part_base, uint32_t nsets, unsigned long long *err,
-                               const PartArgs *part, cudaStream_t st) {
-    if (M == 0) return cudaSuccess;
-    PartArgs p{};
-    if (part) p = *part;
-    k_check_sizes<<<(M + 255) / 256, 256, 0, st>>>(out, M, stride, cap, part_base, nsets, err, p, part != nullptr);
     return cudaGetLastError();
 }
 

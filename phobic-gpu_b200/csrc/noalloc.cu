@@ -175,14 +175,14 @@ extern "C" phobic_status phobic_build_noalloc(const phobic_keys *keys, const pho
         ScanArgs sa{d_count, d_G, d_count, (uint32_t)m, d_tiles, reinterpret_cast<uint32_t *>(d_tiles + tiles), 1,
                     d_err, 0};
         SearchArgs qa{d_desc, d_pb, 1, (uint32_t)m, d_G, 1, d_lowers, d_bkt, d_sorted, nullptr, B, cap, k_max,
-                      d_queue, d_err, d_count};
+                      d_queue, d_err, d_count, P};
         uint64_t kc_index = 0, kc_mask = 0;
         ok = cuda(launch_map_count(keys->kind, ma, plan, s));
         if (ok && take_key_change(n, keys->kind, &kc_index, &kc_mask))
             ok = cuda(launch_change_key(const_cast<void *>(keys->data), kc_index, kc_mask, s));
         ok = ok && cuda(launch_scan(sa, s)) &&
-             cuda(launch_check_sizes(d_G, (uint32_t)m, 1, cap, d_pb, 1, d_err, nullptr, s)) &&
-             cuda(launch_scatter(keys->kind, ma, plan, s)) && cuda(launch_search(qa, sm_count, s));
+             cuda(launch_scatter(keys->kind, ma, plan, s)) && cuda(launch_order(qa, sm_count, s)) &&
+             cuda(launch_search(qa, sm_count, s));
     }
     if (!ok) cudaGetLastError();
     // Bounded wait for everything queued above (also after a failed launch: work queued
