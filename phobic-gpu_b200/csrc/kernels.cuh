@@ -212,9 +212,8 @@ struct SearchShape {
 };
 cudaError_t launch_search(const SearchArgs &a, int sm_count, cudaStream_t st, SearchShape shape = SearchShape{});
 // Default shape when the autotuner's table has no line for a build, fitted to the B200's
-// measurements: bucket pipelines of 8 warps up to 256 partitions, of 4 up to 512, of 2 up
-// to 1024, else one warp per partition; a group only while the groups fit one wave of the
-// group kernel.
+// measurements: bucket pipelines of 8 warps up to 256 partitions, of 4 up to about 3100, else
+// one warp per partition.
 SearchShape search_shape_for(uint32_t partitions, int sm_count);
 size_t search_group_smem(uint32_t buckets, uint32_t cap, int W);
 // First failed bounds check of each kernel file in the checked build (source line, 0 =

@@ -89,8 +89,14 @@ __device__ __forceinline__ uint4 lds128(uint32_t addr) {
     asm volatile("ld.shared.v4.u32 {%0, %1, %2, %3}, [%4];" : "=r"(v.x), "=r"(v.y), "=r"(v.z), "=r"(v.w) : "r"(addr));
     return v;
 }
-__device__ __forceinline__ void red_or(uint32_t addr, uint32_t bit) {
-    asm volatile("red.shared.or.b32 [%0], %1;" ::"r"(addr), "r"(bit) : "memory");
+// The word at addr before `bit` is set in it, where `on` (else 0, and nothing is set).
+__device__ __forceinline__ uint32_t atom_or_if(uint32_t addr, uint32_t bit, bool on) {
+    uint32_t old;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tmov.u32 %0, 0;\n\t"
+        "@p atom.shared.or.b32 %0, [%1], %2;\n\t}"
+        : "=&r"(old) : "r"(addr), "r"(bit), "r"((uint32_t)on) : "memory");
+    return old;
 }
 __device__ __forceinline__ void red_and(uint32_t addr, uint32_t mask) {
     asm volatile("red.shared.and.b32 [%0], %1;" ::"r"(addr), "r"(mask) : "memory");
@@ -100,19 +106,29 @@ __device__ __forceinline__ void red_and(uint32_t addr, uint32_t mask) {
 // as its second).
 __device__ __forceinline__ uint32_t pair_of(uint32_t q) { return (q >> 5) << 3; }
 
-// Sets slot q and its mirror q + ps, each in the two pairs that hold its word.
-__device__ __forceinline__ void mark(uint32_t occ, uint32_t q, uint32_t ps) {
-    const uint32_t a = occ + pair_of(q), bit = 1u << (q & 31), m = q + ps;
-    const uint32_t b = occ + pair_of(m), mbit = 1u << (m & 31);
-    red_or(a, bit);
-    red_or(a - 4, bit);
-    red_or(b, mbit);
-    red_or(b - 4, mbit);
+// The bits of slot q where `on`: its own place (the one that is tested) and, apart from it, the
+// second place of its word and both of its mirror q + ps; predicated, without a branch.
+__device__ __forceinline__ void mark_own(uint32_t at, uint32_t bit, bool on) {
+    asm volatile("{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %2, 0;\n\t@p red.shared.or.b32 [%0], %1;\n\t}" ::"r"(at),
+                 "r"(bit), "r"((uint32_t)on)
+                 : "memory");
 }
-__device__ __forceinline__ bool is_taken(uint32_t occ, uint32_t q) {
-    uint32_t w;
-    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(w) : "r"(occ + pair_of(q)) : "memory");
-    return (w >> (q & 31)) & 1u;
+__device__ __forceinline__ void mark_copies(uint32_t occ, uint32_t q, uint32_t ps, bool on) {
+    const uint32_t m = q + ps;
+    asm volatile(
+        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
+        "@p red.shared.or.b32 [%0+-4], %1;\n\t@p red.shared.or.b32 [%2], %3;\n\t@p red.shared.or.b32 [%2+-4], %3;\n\t}"
+        ::"r"(occ + pair_of(q)), "r"(1u << (q & 31)), "r"(occ + pair_of(m)), "r"(1u << (m & 31)), "r"((uint32_t)on)
+        : "memory");
+}
+__device__ __forceinline__ void mark(uint32_t occ, uint32_t q, uint32_t ps) {
+    mark_own(occ + pair_of(q), 1u << (q & 31), true);
+    mark_copies(occ, q, ps, true);
+}
+__device__ __forceinline__ uint32_t lds32(uint32_t addr) {
+    uint32_t v;
+    asm volatile("ld.shared.u32 %0, [%1];" : "=r"(v) : "r"(addr) : "memory");
+    return v;
 }
 
 // A slot h as the offset search reads it: the byte offset of its pair, 8 * (h >> 5),
@@ -241,22 +257,14 @@ __device__ __noinline__ bool has_duplicate_key(uint2 L, uint32_t s, int lane) {
 // false when two of the lanes hold the same slot.  The slots were free before.  Predicated
 // instructions: the lanes of a bucket mark without a divergent branch.
 __device__ __forceinline__ bool mark_distinct(uint32_t occ, uint32_t q, uint32_t ps, bool on) {
-    const uint32_t a = occ + pair_of(q), bit = 1u << (q & 31), m = q + ps;
-    const uint32_t b = occ + pair_of(m), mbit = 1u << (m & 31);
-    uint32_t old;
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %3, 0;\n\tmov.u32 %0, 0;\n\t"
-        "@p atom.shared.or.b32 %0, [%1], %2;\n\t}"
-        : "=&r"(old) : "r"(a), "r"(bit), "r"((uint32_t)on) : "memory");
+    const uint32_t a = occ + pair_of(q), bit = 1u << (q & 31);
+    const uint32_t old = atom_or_if(a, bit, on);
     if (__any_sync(kFullMask, old & bit)) {
         if (on) red_and(a, ~bit);
         __syncwarp();
         return false;
     }
-    asm volatile(
-        "{\n\t.reg .pred p;\n\tsetp.ne.u32 p, %4, 0;\n\t"
-        "@p red.shared.or.b32 [%0+-4], %1;\n\t@p red.shared.or.b32 [%2], %3;\n\t@p red.shared.or.b32 [%2+-4], %3;\n\t}"
-        ::"r"(a), "r"(bit), "r"(b), "r"(mbit), "r"((uint32_t)on) : "memory");
+    mark_copies(occ, q, ps, on);
     __syncwarp();
     return true;
 }
@@ -285,14 +293,9 @@ __device__ __forceinline__ uint32_t lane_key(uint32_t s, int lane) {
 // lane_key loads it.  The warp hashes 32 / S pilot counters at once (lane t * S + i holds key i
 // under counter k0 + t) into hs and tests them in counter order, so a counter that fails costs
 // no new hash.  Same result as trying k = 0, 1, 2, ... one at a time (search.comp:105-124).
-// With MARK the slots are marked and *pilot written; without, nothing is marked and the bucket
-// pipeline gets the counter, the offset and (lanes < s) the lane's slot in *k_out, *o_out,
-// *q_out.
-template <int S, bool MARK = true>
+template <int S>
 __device__ __forceinline__ uint32_t place_batched(const WarpSmem &ws, uint2 L, uint32_t s, const ScanRange &sr,
-                                                  FastMod fm, uint32_t k_lim, int lane, uint32_t *pilot,
-                                                  uint32_t *k_out = nullptr, uint32_t *o_out = nullptr,
-                                                  uint32_t *q_out = nullptr) {
+                                                  FastMod fm, uint32_t k_lim, int lane, uint32_t *pilot) {
     constexpr uint32_t G = 32 / S;
     const uint32_t hs_sa = (uint32_t)__cvta_generic_to_shared(ws.hs);
     const bool mine = lane < (int)s;
@@ -316,30 +319,138 @@ __device__ __forceinline__ uint32_t place_batched(const WarpSmem &ws, uint2 L, u
             if (o == kNone) continue;
             uint32_t q = unpack_slot(ws.hs[S * u + (mine ? (uint32_t)lane : 0u)]) + o;
             q = q >= sr.ps ? q - sr.ps : q;
-            const bool on = mine && PHB_CHECK(!mine || q < sr.ps);
-            if constexpr (MARK) {
-                if (!mark_distinct(ws.occ, q, sr.ps, on)) continue;
-                *pilot = o + sr.ps * (k0 + u);
-            } else {
-                if (!slots_distinct(ws.scr, q, on)) continue;
-                *k_out = k0 + u;
-                *o_out = o;
-                *q_out = q;
-            }
+            if (!mark_distinct(ws.occ, q, sr.ps, mine && PHB_CHECK(!mine || q < sr.ps))) continue;
+            *pilot = o + sr.ps * (k0 + u);
             return PHOBIC_OK;
         }
     }
 }
 
 // place_batched for any bucket of at most 32 keys.
-template <bool MARK>
 __device__ __forceinline__ uint32_t place_any(const WarpSmem &ws, uint2 L, uint32_t s, const ScanRange &sr, FastMod fm,
-                                              uint32_t k_lim, int lane, uint32_t *pilot, uint32_t *k_out = nullptr,
-                                              uint32_t *o_out = nullptr, uint32_t *q_out = nullptr) {
-    if (s <= 4) return place_batched<4, MARK>(ws, L, s, sr, fm, k_lim, lane, pilot, k_out, o_out, q_out);
-    if (s <= 8) return place_batched<8, MARK>(ws, L, s, sr, fm, k_lim, lane, pilot, k_out, o_out, q_out);
-    if (s <= 16) return place_batched<16, MARK>(ws, L, s, sr, fm, k_lim, lane, pilot, k_out, o_out, q_out);
-    return place_batched<32, MARK>(ws, L, s, sr, fm, k_lim, lane, pilot, k_out, o_out, q_out);
+                                              uint32_t k_lim, int lane, uint32_t *pilot) {
+    if (s <= 4) return place_batched<4>(ws, L, s, sr, fm, k_lim, lane, pilot);
+    if (s <= 8) return place_batched<8>(ws, L, s, sr, fm, k_lim, lane, pilot);
+    if (s <= 16) return place_batched<16>(ws, L, s, sr, fm, k_lim, lane, pilot);
+    return place_batched<32>(ws, L, s, sr, fm, k_lim, lane, pilot);
+}
+
+// ------------------------------------------------------------------ low-latency search
+//
+// The group kernel's warps are few, so what counts there is the length of one try's chain, not
+// its instructions: all NR rounds of a partition of at most 1024 NR offsets are in flight at
+// once, the collision test runs beside them, and the smallest offset comes from one warp-wide
+// minimum.
+
+// This lane's windows in all NR rounds (bad[r] bit i: offset 1024 r + 32 lane + i is taken) of a
+// bucket of s keys whose packed slots start at the shared address hs, S of them (S = 4 or 8), or
+// s padded to a multiple of 4 (S = 16 or 32).  For S = 4 it returns whether two of the keys share
+// a slot.
+template <int S, int NR>
+__device__ __forceinline__ bool all_windows(const WarpSmem &ws, uint32_t hs, uint32_t s, const ScanRange &sr, int lane,
+                                            uint32_t (&bad)[NR]) {
+    const uint32_t lane_sa = ws.occ + 8u * lane;
+#pragma unroll
+    for (int r = 0; r < NR; r++) bad[r] = r == NR - 1 ? sr.last_dead : 0u;
+    auto quad = [&](uint4 v, bool half) {
+        const uint32_t x[4] = {v.x, v.y, v.z, v.w};
+#pragma unroll
+        for (int i = 0; i < 4; i += 2) {
+            if (i == 2 && half) break;
+            const uint32_t a = lane_sa + (x[i] >> 5), b = lane_sa + (x[i + 1] >> 5);
+            bad[0] |= window_at<0>(ws, a, x[i]) | window_at<0>(ws, b, x[i + 1]);
+            if constexpr (NR > 1) bad[1] |= window_at<256>(ws, a, x[i]) | window_at<256>(ws, b, x[i + 1]);
+            if constexpr (NR > 2) bad[2] |= window_at<512>(ws, a, x[i]) | window_at<512>(ws, b, x[i + 1]);
+        }
+    };
+    if constexpr (S == 4) {
+        const uint4 v = lds128(hs);
+        quad(v, s <= 2);
+        return (s > 1 && v.x == v.y) || (s > 2 && (v.x == v.z || v.y == v.z)) ||
+               (s > 3 && (v.x == v.w || v.y == v.w || v.z == v.w));
+    } else if constexpr (S == 8) {
+        quad(lds128(hs), false);
+        quad(lds128(hs + 16), s <= S - 2);
+    } else {
+        const uint32_t hs_end = hs + 4 * s;
+#pragma unroll 2
+        for (uint32_t q = hs; q < hs_end; q += 16) quad(lds128(q), false);
+    }
+    return false;
+}
+
+// The warp's smallest free offset in these windows (kNone: none).
+template <int NR>
+__device__ __forceinline__ uint32_t smallest_offset(const uint32_t (&bad)[NR], int lane) {
+    uint32_t open = ~bad[NR - 1], at = 1024u * (NR - 1);  // the lane's first round with a free offset
+#pragma unroll
+    for (int r = NR - 2; r >= 0; r--) {
+        const bool here = bad[r] != kFullMask;
+        open = here ? ~bad[r] : open;
+        at = here ? 1024u * r : at;
+    }
+    return __reduce_min_sync(kFullMask, open ? at + 32u * lane + __ffs(open) - 1 : kNone);
+}
+
+// A search of the bucket pipeline: pilot counter, offset, the lane's slot under that counter
+// before the offset (lanes below the bucket's size), and the windows it was found in.
+template <int NR>
+struct Seek {
+    uint32_t kb, k, o, h;
+    uint32_t bad[NR ? NR : 1];
+};
+
+// The search of place_batched as the bucket pipeline runs it: nothing is marked, and it can be
+// resumed.  Finds the smallest pilot counter >= k, then the smallest offset, that the bitmap
+// allows; kb is the first counter of the batch whose slots hs holds (kNone: none yet), so a
+// second call with the same k tests that counter again without a hash.  NR = 0: any number of
+// rounds, one after the other.
+template <int S, int NR>
+__device__ __forceinline__ uint32_t seek_batched(const WarpSmem &ws, uint32_t *hs, uint2 L, uint32_t s,
+                                                 const ScanRange &sr, FastMod fm, uint32_t k_lim, int lane, Seek<NR> *f) {
+    constexpr uint32_t G = 32 / S;
+    const uint32_t hs_sa = (uint32_t)__cvta_generic_to_shared(hs);
+    const bool mine = lane < (int)s;
+#pragma unroll 1
+    for (;; ++f->k) {
+        if (f->k >= k_lim) return PHOBIC_ERR_SEARCH_LIMIT;
+        const uint32_t u = f->k % G;
+        if (f->k - u != f->kb) {  // u = 0: a batch is entered at its first counter
+            if (f->k == kDupCheckAt && s > 1 && has_duplicate_key(L, s, lane)) return PHOBIC_ERR_DUPLICATE_KEY;
+            f->kb = f->k;
+            const uint32_t hk = pack_slot(fm.mod(pilot_hash(L.x, L.y, f->k + (uint32_t)lane / S)));
+            __syncwarp();
+            hs[lane] = hk;
+        }
+        __syncwarp();
+        const uint32_t own = hs[S * u + (mine ? (uint32_t)lane : 0u)];
+        bool meet = false;
+        if constexpr (NR > 0) meet = all_windows<S, NR>(ws, hs_sa + 4 * S * u, s, sr, lane, f->bad);
+        else if constexpr (S <= 8) f->o = scan_small<S>(ws, hs_sa + 4 * S * u, s, sr, lane);
+        else f->o = scan_quads(ws, hs_sa + 4 * S * u, s, sr, lane);
+        f->h = unpack_slot(own);
+        if constexpr (S == 4 && NR > 0) {
+            f->o = smallest_offset<NR>(f->bad, lane);
+        } else {
+            // Two keys on one slot: their bits meet in the warp's collision scratch (left clear).
+            const bool on = mine && s > 1 && PHB_CHECK(f->h < sr.ps);
+            const uint32_t bit = 1u << (f->h & 31), at = (uint32_t)__cvta_generic_to_shared(ws.scr) + 4 * (f->h >> 5);
+            const uint32_t old = atom_or_if(at, bit, on) & bit;
+            if constexpr (NR > 0) f->o = smallest_offset<NR>(f->bad, lane);
+            meet = __any_sync(kFullMask, old);
+            if (on) ws.scr[f->h >> 5] = 0;
+            __syncwarp();
+        }
+        if (!meet && f->o != kNone) return PHOBIC_OK;
+    }
+}
+template <int NR>
+__device__ __forceinline__ uint32_t seek_any(const WarpSmem &ws, uint32_t *hs, uint2 L, uint32_t s, const ScanRange &sr,
+                                             FastMod fm, uint32_t k_lim, int lane, Seek<NR> *f) {
+    if (s <= 4) return seek_batched<4, NR>(ws, hs, L, s, sr, fm, k_lim, lane, f);
+    if (s <= 8) return seek_batched<8, NR>(ws, hs, L, s, sr, fm, k_lim, lane, f);
+    if (s <= 16) return seek_batched<16, NR>(ws, hs, L, s, sr, fm, k_lim, lane, f);
+    return seek_batched<32, NR>(ws, hs, L, s, sr, fm, k_lim, lane, f);
 }
 
 // One bucket of more than 32 keys (a few per partition).  Each try hashes chunk by chunk and
@@ -444,7 +555,7 @@ __device__ __forceinline__ uint32_t search_partition(const SearchArgs &a, uint32
             if (s_next <= 32) L_next = so[(sc & 0xFFFFu) + lane_key(s_next, lane)];
         }
         uint32_t pilot = 0;
-        const uint32_t st_code = s <= 32 ? place_any<true>(ws, L, s, sr, fm, k_lim, lane, &pilot)
+        const uint32_t st_code = s <= 32 ? place_any(ws, L, s, sr, fm, k_lim, lane, &pilot)
                                          : place_large(ws, so + st, s, sr, fm, k_lim, lane, &pilot);
         if (st_code != PHOBIC_OK) return st_code;
         if (lane == 0 && PHB_CHECK(b < a.buckets)) pil[(size_t)b * pstride] = pilot;
@@ -471,16 +582,18 @@ __device__ __forceinline__ void group_bar(uint32_t id, uint32_t threads) {
     asm volatile("bar.sync %0, %1;" ::"r"(id), "r"(threads) : "memory");
 }
 
+// The turn of the bucket pipeline: a hardware barrier per warp that its predecessor arrives at
+// and the warp waits on (64 threads).
+__device__ __forceinline__ void turn_wait(uint32_t id) { asm volatile("bar.sync %0, 64;" ::"r"(id) : "memory"); }
+__device__ __forceinline__ void turn_pass(uint32_t id) { asm volatile("bar.arrive %0, 64;" ::"r"(id) : "memory"); }
+
 // Per-warp scratch of warps 1..W-1 of a group (warp 0 uses its place in carve()).
 __host__ __device__ __forceinline__ size_t group_extra_words(uint32_t cap) {
     return ((size_t)kHsWords + scr_words(cap) + 3) & ~size_t(3);
 }
-// Exchange words: [2 parities][W] outcomes, the control words (job, nonempty, committed,
-// status), and the bucket pipeline's results: [W] (code << 24 | k, offset) pairs and [W][32]
-// slots (padded).
-__host__ __device__ __forceinline__ size_t group_xch_words(int W) {
-    return ((size_t)2 * W + 4 + 2 * (size_t)W + 32 * (size_t)W + 3) & ~size_t(3);
-}
+// Exchange words: [2 parities][W] outcomes of the k-split steps and the control words (job,
+// nonempty, status; padded).
+__host__ __device__ __forceinline__ size_t group_xch_words(int W) { return ((size_t)2 * W + 4 + 3) & ~size_t(3); }
 __host__ __device__ __forceinline__ size_t group_words(uint32_t B, uint32_t cap, int W) {
     return warp_words(B, cap) + (size_t)(W - 1) * group_extra_words(cap) + group_xch_words(W);
 }
@@ -503,32 +616,36 @@ __device__ __forceinline__ uint32_t try_small(const WarpSmem &ws, uint32_t s, co
     return kTryFound;
 }
 
-// One try of pilot counter k for a bucket of more than 32 keys read from src: the
-// chunked collision test and offset scan of place_large.
-__device__ __forceinline__ uint32_t try_large(const WarpSmem &ws, const uint2 *src, uint32_t s, const ScanRange &sr,
+// Keys i = 32 c + lane of a bucket of at most 32 C keys (zero past its end).
+template <int C>
+__device__ __forceinline__ void load_keys(uint2 (&key)[C], const uint2 *src, uint32_t s, int lane) {
+#pragma unroll
+    for (int c = 0; c < C; c++) key[c] = 32 * c + lane < (int)s ? src[32 * c + lane] : make_uint2(0, 0);
+}
+
+// One try of pilot counter k for a bucket of more than 32 keys: all chunks are hashed side by side
+// (the collision test of place_large, without its early end: here the chain counts).
+template <int C>
+__device__ __forceinline__ uint32_t try_large(const WarpSmem &ws, const uint2 (&key)[C], uint32_t s, const ScanRange &sr,
                                               FastMod fm, uint32_t k, int lane, uint32_t *o_out) {
-    const uint32_t padded = (s + 3) & ~3u;
+    uint32_t h[C], old = 0;
+#pragma unroll
+    for (int c = 0; c < C; c++) h[c] = fm.mod(pilot_hash(key[c].x, key[c].y, k));
+#pragma unroll
+    for (int c = 0; c < C; c++)
+        if (32 * c + lane < (int)s && PHB_CHECK(h[c] < sr.ps))
+            old |= atomicOr(&ws.scr[h[c] >> 5], 1u << (h[c] & 31)) & (1u << (h[c] & 31));
+    const bool meet = __any_sync(kFullMask, old);
+#pragma unroll
+    for (int c = 0; c < C; c++)
+        if (32 * c + lane < (int)s && PHB_CHECK(h[c] < sr.ps)) ws.scr[h[c] >> 5] = 0;
+    __syncwarp();
+    if (meet) return kTryNone;
+#pragma unroll
+    for (int c = 0; c < C; c++)  // past the end: any slot of the bucket, as padding
+        if (32 * c < (int)s) ws.hs[32 * c + lane] = pack_slot(__shfl_sync(kFullMask, h[c], 32 * c + lane < (int)s ? lane : 0));
+    __syncwarp();
     const uint32_t hs_sa = (uint32_t)__cvta_generic_to_shared(ws.hs);
-    bool dup = false;
-    uint32_t done = 0;
-    for (uint32_t c0 = 0; c0 < s && !dup; c0 += 32) {
-        const uint32_t i = c0 + lane;
-        bool d = false;
-        if (i < s) {
-            const uint2 key = src[i];
-            const uint32_t h = fm.mod(pilot_hash(key.x, key.y, k));
-            ws.hs[i] = pack_slot(h);
-            const uint32_t bit = 1u << (h & 31);
-            d = PHB_CHECK(h < sr.ps) && (atomicOr(&ws.scr[h >> 5], bit) & bit) != 0;
-        }
-        dup = __any_sync(kFullMask, d);
-        done = c0 + 32;
-    }
-    for (uint32_t i = lane; i < s && i < done; i += 32) ws.scr[unpack_slot(ws.hs[i]) >> 5] = 0;
-    __syncwarp();
-    if (dup) return kTryNone;
-    if (s + lane < padded) ws.hs[s + lane] = ws.hs[0];
-    __syncwarp();
     const uint32_t o = scan_quads(ws, hs_sa, s, sr, lane);
     __syncwarp();
     if (o == kNone) return kTryNone;
@@ -547,39 +664,156 @@ __device__ __noinline__ bool has_duplicate_key_src(const uint2 *src, uint32_t s,
     return __any_sync(kFullMask, d);
 }
 
-// Marks the slots (h_i + o) mod ps of the bucket's keys at pilot counter k.
-__device__ __forceinline__ void mark_bucket(const WarpSmem &ws, uint2 L, const uint2 *src, uint32_t s, uint32_t ps,
-                                            FastMod fm, uint32_t k, uint32_t o, int lane) {
-    if (s <= 32) {
-        if (lane < (int)s) {
-            uint32_t q = fm.mod(pilot_hash(L.x, L.y, k)) + o;
-            q = q >= ps ? q - ps : q;
-            if (PHB_CHECK(q < ps)) mark(ws.occ, q, ps);
+// One bucket in k-split steps by all W warps of a group; C = 1 for at most 32 keys.  Marks the
+// winning slots (every warp: the marks are idempotent).  Returns a status; *pilot when it is OK.
+template <int W, int C>
+__device__ __forceinline__ uint32_t ksplit_bucket(const WarpSmem &ws, const uint2 *src, uint32_t s, const ScanRange &sr,
+                                                  FastMod fm, uint32_t k_lim, uint32_t *xch, uint32_t *par, int w,
+                                                  int lane, uint32_t bar_id, uint32_t *pilot) {
+    uint2 key[C];
+    if constexpr (C == 1) key[0] = src[lane_key(s, lane)];
+    else load_keys(key, src, s, lane);
+#pragma unroll 1
+    for (uint32_t k0 = 0;; k0 += W) {
+        const uint32_t k = k0 + w;
+        uint32_t code = kTryNone, o = 0;
+        if (k >= k_lim) code = kTryLimit;
+        else if (k == kDupCheckAt && s > 1 && (C == 1 ? has_duplicate_key(key[0], s, lane) : has_duplicate_key_src(src, s, lane)))
+            code = kTryDup;
+        else if constexpr (C == 1) code = try_small(ws, s, sr, fm.mod(pilot_hash(key[0].x, key[0].y, k)), lane, &o);
+        else code = try_large<C>(ws, key, s, sr, fm, k, lane, &o);
+        if (lane == 0) xch[*par * W + w] = (code << 16) | (o & 0xFFFFu);
+        group_bar(bar_id, 32 * W);
+        uint32_t win = kTryNone << 16, v = 0;
+#pragma unroll
+        for (int i = W - 1; i >= 0; i--) {
+            const uint32_t x = xch[*par * W + i];
+            if ((x >> 16) != kTryNone) win = x, v = i;
         }
-    } else {
-        for (uint32_t i = lane; i < s; i += 32) {
-            const uint2 key = src[i];
-            uint32_t q = fm.mod(pilot_hash(key.x, key.y, k)) + o;
-            q = q >= ps ? q - ps : q;
-            if (PHB_CHECK(q < ps)) mark(ws.occ, q, ps);
+        *par ^= 1u;
+        const uint32_t wcode = win >> 16;
+        if (wcode == kTryNone) continue;
+        if (wcode != kTryFound) return wcode == kTryDup ? PHOBIC_ERR_DUPLICATE_KEY : PHOBIC_ERR_SEARCH_LIMIT;
+        const uint32_t kw = k0 + v, ow = win & 0xFFFFu;
+#pragma unroll
+        for (int c = 0; c < C; c++) {
+            if (32 * c + lane < (int)s) {
+                uint32_t q = fm.mod(pilot_hash(key[c].x, key[c].y, kw)) + ow;
+                q = q >= sr.ps ? q - sr.ps : q;
+                if (PHB_CHECK(q < sr.ps)) mark(ws.occ, q, sr.ps);
+            }
         }
+        __syncwarp();
+        *pilot = ow + sr.ps * kw;
+        return PHOBIC_OK;
     }
-    __syncwarp();
+}
+
+// The bucket pipeline of a group from bucket `first` on (see k_search_group); NR as in
+// seek_batched.
+template <int W, int NR>
+__device__ __forceinline__ void pipeline(const WarpSmem &ws, const uint2 *so, const ScanRange &sr, FastMod fm,
+                                         uint32_t k_lim, uint32_t first, uint32_t nonempty, int w, int lane,
+                                         uint32_t turn_id, uint32_t next_id, volatile uint32_t *status,
+                                         uint32_t *pil, size_t pstride) {
+    // Ahead of the warp's bucket: the schedule of its third next bucket is read, the keys of the
+    // second next one, and the first batch of slots of the next one is hashed, into one half of hs,
+    // while the warp's bucket waits for its turn with the other.
+    struct Ahead {
+        uint32_t sc, s;
+        uint2 L;
+    } n1{0, 0, make_uint2(0, 0)}, n2 = n1;
+    uint32_t sc3 = 0, end3 = 0;
+    auto read = [&](uint32_t j) {
+        if (j >= nonempty) return;
+        sc3 = ws.sched[j];
+        end3 = ws.sched[j + 1];
+    };
+    auto fetch = [&](uint32_t j) {
+        if (j >= nonempty) return;
+        n2.sc = sc3;
+        n2.s = (end3 - sc3) & 0xFFFFu;
+        n2.L = so[(sc3 & 0xFFFFu) + lane_key(n2.s, lane)];
+    };
+    auto hash_first = [&](uint32_t *hs) {
+        hs[lane] = pack_slot(fm.mod(pilot_hash(n1.L.x, n1.L.y, (uint32_t)lane / counter_lanes(n1.s))));
+    };
+    read(first + w);
+    fetch(first + w);
+    n1 = n2;
+    read(first + w + W);
+    fetch(first + w + W);
+    read(first + w + 2 * W);
+    uint32_t half = 0;
+    if (first + w < nonempty) hash_first(ws.hs);
+#pragma unroll 1
+    for (uint32_t j = first + w; j < nonempty; j += W, half ^= 32u) {
+        const uint32_t s = n1.s, b = n1.sc >> 16;
+        const uint2 L = n1.L;
+        n1 = n2;
+        fetch(j + 2 * W);
+        read(j + 3 * W);
+        Seek<NR> f;
+        f.kb = f.k = f.o = f.h = 0;
+        uint32_t st = *status, q = 0, at = 0, bit = 0;
+        bool turn = false, seek = st == PHOBIC_OK, on = false;
+#pragma unroll 1
+        for (;;) {
+            if (seek) st = seek_any<NR>(ws, ws.hs + half, L, s, sr, fm, k_lim, lane, &f);
+            on = lane < (int)s && st == PHOBIC_OK && PHB_CHECK(f.h < sr.ps && f.o < sr.ps);
+            q = f.h + f.o;
+            q = q >= sr.ps ? q - sr.ps : q;
+            at = on ? ws.occ + pair_of(q) : ws.occ;
+            bit = on ? 1u << (q & 31) : 0u;
+            if (!turn) {
+                if (j + W < nonempty) hash_first(ws.hs + (half ^ 32u));
+                if (j > first) turn_wait(turn_id);
+                turn = true;
+            }
+            if (!__any_sync(kFullMask, lds32(at) & bit)) break;
+            // An earlier bucket took a slot since: the next free offset of the same windows, or
+            // the next counter.
+            seek = true;
+            if constexpr (NR > 0) {
+#pragma unroll
+                for (int r = 0; r < NR; r++)
+                    if (f.o >> 5 == (uint32_t)(32 * r + lane)) f.bad[r] |= 1u << (f.o & 31);
+                f.o = smallest_offset<NR>(f.bad, lane);
+                seek = f.o == kNone;
+                if (seek) ++f.k;
+            }
+        }
+        mark_own(at, bit, on);
+        if (st != PHOBIC_OK && lane == 0 && *status == PHOBIC_OK) *status = st;
+        __syncwarp();
+        if (j + 1 < nonempty) turn_pass(next_id);
+        mark_copies(ws.occ, q, sr.ps, on);
+        if (st == PHOBIC_OK && lane == 0) pil[(size_t)b * pstride] = f.o + sr.ps * f.k;
+    }
 }
 
 // Group kernel: kSearchWarps / W groups per CTA, each a persistent searcher over the
 // partition queue; all W warps of a group search a partition's buckets in k-split steps.
 // Small builds leave most SMs idle, so the group kernel is not held to the one-warp
 // kernel's 4 CTAs per SM (64 registers): 2 CTAs per SM keep it free of spills.
-// Bucket pipeline (PIPE): for buckets of at most 32 keys (the tail of the search order),
-// warp w searches bucket j + w completely (smallest k, then smallest o) on the bitmap as it
-// stands, without marking.  Warp 0 then commits the W results in order: a result is kept
-// while its slots are still free after the results before it were marked.  That keeps the
-// sequential answer: the bitmap only gains occupied slots, so a (k, o) valid on the later
-// state was valid on the earlier one, and the smallest valid pair on the earlier state, if
-// still valid, is the smallest on the later one.  A pilot limit or duplicate keys found on the
-// earlier state hold on the later one too.  The first result that conflicts is searched again
-// in the next step.
+// Bucket pipeline (PIPE): the buckets of at most 32 keys (the tail of the search order) go to the
+// warps in turn.  A warp searches its bucket (smallest k, then smallest o) on the bitmap as it
+// stands, without marking, and then waits for its turn: the arrival of the warp that holds the
+// bucket before.  On its turn it tests its slots where the earlier buckets marked them, takes the
+// next free offset of the windows it saw (then the next counters) while one of them is taken, marks
+// them, and passes the turn on; the
+// bitmap's copies of the marks (second words of pairs, mirrors), which only searches read, follow
+// after.  That keeps the sequential answer: the bitmap only gains occupied slots, so what was
+// rejected stays rejected, a pair that a search found without some marks fails the test, and the
+// first pair that passes it is the smallest.  A pilot limit or duplicate keys found on an earlier
+// state hold on the later one too; the first bucket in order that fails sets the partition's
+// status, and the turns go round without searches from then on.
+// From bucket to bucket the chain is a hardware barrier (34 cycles from arrival to wake-up; a
+// polled word takes 120), a look at the slots, a vote and one reduction (25 cycles each).
+// Against the step pipeline before it (W searches, barrier, commits by one warp up to the first
+// conflict, barrier; keys loaded at the start of a step) the search takes 59 against 143 us for
+// 1000 keys, 104 against 205 for 98,765 (lambda 6, P 2048), 127 against 264 for 10^6 (lambda 5).
+// With 3 CTAs per SM (80 registers, spills) it is 12 to 20 % slower.
 template <int W, bool PIPE>
 __global__ void __launch_bounds__(kSearchWarps * 32, 2) k_search_group(SearchArgs a) {
     extern __shared__ __align__(16) uint32_t smem[];
@@ -594,9 +828,9 @@ __global__ void __launch_bounds__(kSearchWarps * 32, 2) k_search_group(SearchArg
         ws.scr = ws.hs + kHsWords;
     }
     uint32_t *xch = gbase + warp_words(a.buckets, a.cap) + (size_t)(W - 1) * group_extra_words(a.cap);
-    uint32_t *ctl = xch + 2 * W;  // [0] job, [1] nonempty, [2] committed, [3] status
-    uint32_t *pres = ctl + 4;     // [W] pairs: code << 24 | k, offset
-    uint32_t *pslots = pres + 2 * W;  // [W][32] slots of each warp's result
+    uint32_t *ctl = xch + 2 * W;  // [0] job, [1] nonempty, [2] status of the pipeline
+    const uint32_t turn_id = 1 + kSearchWarps / W + (uint32_t)warp;  // this warp's turn; group barriers before
+    const uint32_t next_id = 1 + kSearchWarps / W + (uint32_t)(grp * W + (w + 1) % W);
     uint32_t par = 0;
     for (;;) {
         if (w == 0 && lane == 0) ctl[0] = atomicAdd(a.queue, 1u);
@@ -616,6 +850,7 @@ __global__ void __launch_bounds__(kSearchWarps * 32, 2) k_search_group(SearchArg
             }
             if (ctl1 == 0) ctl1 = 0xFFFFFFFFu;
             ctl[1] = ctl1;
+            ctl[2] = PHOBIC_OK;
         }
         group_bar(bar_id, bar_n);
         const uint32_t nonempty = ctl[1];
@@ -628,95 +863,36 @@ __global__ void __launch_bounds__(kSearchWarps * 32, 2) k_search_group(SearchArg
             load_partition(a, gbase, ws0, base, ps, nonempty, (uint32_t)(32 * w + lane), bar_n);
             if (w > 0)
                 for (uint32_t i = lane; i < scr_words(a.cap); i += 32) ws.scr[i] = 0;
+            // The keys of the large buckets, which come first, into L1 (16 keys a line).
+            const uint32_t line = 16 * (uint32_t)(32 * w + lane);
+            if (line < ps) asm volatile("{\n\t.reg .b32 t;\n\tld.global.u32 t, [%0];\n\t}" ::"l"(so + line));
             group_bar(bar_id, bar_n);
             const FastMod fm = FastMod::make(ps);
             const ScanRange sr = ScanRange::make(ps, lane);
             uint32_t k_lim = 0x80000000u / ps;
             if (k_lim > a.k_max) k_lim = a.k_max;
             uint32_t err = PHOBIC_OK;
-            for (uint32_t j = 0; j < nonempty && err == PHOBIC_OK; j++) {
+            uint32_t j = 0;
+            for (; j < nonempty && err == PHOBIC_OK; j++) {
                 const uint32_t sc = ws.sched[j];
-                const uint32_t b = sc >> 16, st = sc & 0xFFFFu;
-                const uint32_t s = (ws.sched[j + 1] - sc) & 0xFFFFu;
-                const uint2 *src = so + st;
-                if (PIPE && s <= 32) {  // every later bucket is as small (search order: size descending)
-                    const uint32_t jw = j + w;
-                    if (jw < nonempty) {
-                        const uint32_t scw = ws.sched[jw];
-                        const uint32_t sw = (ws.sched[jw + 1] - scw) & 0xFFFFu;
-                        const uint2 Lw = so[(scw & 0xFFFFu) + lane_key(sw, lane)];
-                        uint32_t kk = 0, o = 0, q = 0;
-                        const uint32_t st = place_any<false>(ws, Lw, sw, sr, fm, k_lim, lane, nullptr, &kk, &o, &q);
-                        const uint32_t code = st == PHOBIC_OK                  ? kTryFound
-                                              : st == PHOBIC_ERR_DUPLICATE_KEY ? kTryDup
-                                                                               : kTryLimit;
-                        if (code == kTryFound && lane < (int)sw) pslots[32 * w + lane] = q;
-                        if (lane == 0) {
-                            pres[2 * w] = (code << 24) | (kk & 0xFFFFFFu);
-                            pres[2 * w + 1] = o;
-                        }
-                    }
-                    group_bar(bar_id, bar_n);
-                    if (w == 0) {
-                        uint32_t committed = 0, e = PHOBIC_OK;
-                        for (uint32_t v = 0; v < (uint32_t)W && j + v < nonempty; v++) {
-                            const uint32_t r0 = pres[2 * v], rcode = r0 >> 24;
-                            if (rcode != kTryFound) {
-                                e = rcode == kTryDup ? PHOBIC_ERR_DUPLICATE_KEY : PHOBIC_ERR_SEARCH_LIMIT;
-                                break;
-                            }
-                            const uint32_t scv = ws.sched[j + v], bv = scv >> 16;
-                            const uint32_t sv = (ws.sched[j + v + 1] - scv) & 0xFFFFu;
-                            const bool mine = lane < (int)sv;
-                            const uint32_t q = mine ? pslots[32 * v + lane] : 0u;
-                            const bool on = mine && PHB_CHECK(!mine || q < ps);
-                            if (__any_sync(kFullMask, on && is_taken(ws.occ, q))) break;  // searched again next step
-                            if (on) mark(ws.occ, q, ps);
-                            __syncwarp();
-                            if (lane == 0 && PHB_CHECK(bv < a.buckets))
-                                pil[(size_t)bv * pstride] = pres[2 * v + 1] + ps * (r0 & 0xFFFFFFu);
-                            committed++;
-                        }
-                        if (lane == 0) {
-                            ctl[2] = committed;
-                            ctl[3] = e;
-                        }
-                    }
-                    group_bar(bar_id, bar_n);
-                    err = ctl[3];
-                    j += ctl[2];
-                    j--;  // the loop's increment
-                    continue;
-                }
-                const uint2 L = s <= 32 ? src[lane_key(s, lane)] : make_uint2(0, 0);
-                for (uint32_t k0 = 0;; k0 += W) {
-                    const uint32_t k = k0 + w;
-                    uint32_t code = kTryNone, o = 0;
-                    if (k >= k_lim) code = kTryLimit;
-                    else if (k == kDupCheckAt && s > 1 &&
-                             (s <= 32 ? has_duplicate_key(L, s, lane) : has_duplicate_key_src(src, s, lane)))
-                        code = kTryDup;
-                    else code = s <= 32 ? try_small(ws, s, sr, fm.mod(pilot_hash(L.x, L.y, k)), lane, &o)
-                                        : try_large(ws, src, s, sr, fm, k, lane, &o);
-                    if (lane == 0) xch[par * W + w] = (code << 16) | (o & 0xFFFFu);
-                    group_bar(bar_id, bar_n);
-                    uint32_t win = kTryNone << 16, v = 0;
-                    for (; v < (uint32_t)W; v++) {
-                        win = xch[par * W + v];
-                        if ((win >> 16) != kTryNone) break;
-                    }
-                    par ^= 1u;
-                    const uint32_t wcode = win >> 16;
-                    if (wcode == kTryNone) continue;
-                    if (wcode == kTryFound) {
-                        const uint32_t kw = k0 + v, ow = win & 0xFFFFu;
-                        mark_bucket(ws, L, src, s, ps, fm, kw, ow, lane);
-                        if (w == 0 && lane == 0 && PHB_CHECK(b < a.buckets)) pil[(size_t)b * pstride] = ow + ps * kw;
-                    } else {
-                        err = wcode == kTryDup ? PHOBIC_ERR_DUPLICATE_KEY : PHOBIC_ERR_SEARCH_LIMIT;
-                    }
-                    break;
-                }
+                const uint32_t b = sc >> 16, s = (ws.sched[j + 1] - sc) & 0xFFFFu;
+                const uint2 *src = so + (sc & 0xFFFFu);
+                if (PIPE && s <= 32) break;  // every later bucket is as small (search order: size descending)
+                uint32_t pilot = 0;
+                if (s <= 32) err = ksplit_bucket<W, 1>(ws, src, s, sr, fm, k_lim, xch, &par, w, lane, bar_id, &pilot);
+                else if (s <= 64) err = ksplit_bucket<W, 2>(ws, src, s, sr, fm, k_lim, xch, &par, w, lane, bar_id, &pilot);
+                else if (s <= 128) err = ksplit_bucket<W, 4>(ws, src, s, sr, fm, k_lim, xch, &par, w, lane, bar_id, &pilot);
+                else err = ksplit_bucket<W, 8>(ws, src, s, sr, fm, k_lim, xch, &par, w, lane, bar_id, &pilot);
+                if (err == PHOBIC_OK && w == 0 && lane == 0 && PHB_CHECK(b < a.buckets)) pil[(size_t)b * pstride] = pilot;
+            }
+            if (PIPE && err == PHOBIC_OK && j < nonempty) {
+                volatile uint32_t *status = ctl + 2;
+                if (sr.rounds == 1) pipeline<W, 1>(ws, so, sr, fm, k_lim, j, nonempty, w, lane, turn_id, next_id, status, pil, pstride);
+                else if (sr.rounds == 2) pipeline<W, 2>(ws, so, sr, fm, k_lim, j, nonempty, w, lane, turn_id, next_id, status, pil, pstride);
+                else if (sr.rounds == 3) pipeline<W, 3>(ws, so, sr, fm, k_lim, j, nonempty, w, lane, turn_id, next_id, status, pil, pstride);
+                else pipeline<W, 0>(ws, so, sr, fm, k_lim, j, nonempty, w, lane, turn_id, next_id, status, pil, pstride);
+                group_bar(bar_id, bar_n);
+                err = *status;
             }
             if (err != PHOBIC_OK && w == 0 && lane == 0) report_error(&a.err[s_idx], p, err);
         }
@@ -787,16 +963,16 @@ static cudaError_t launch_group(const SearchArgs &a, int sm_count, cudaStream_t 
 }
 
 SearchShape search_shape_for(uint32_t partitions, int sm_count) {
-    // Measured on a B200 (the autotuner's ladder, three key sets per size, six parameter
-    // sets): bucket pipelines of 8 warps are fastest up to 256 partitions, of 4 warps up to
-    // 512, of 2 warps up to 1024; one warp per partition beyond.  A group must fit one wave
-    // of the group kernel (2 CTAs of kSearchWarps warps per SM).
-    const uint64_t wave = (uint64_t)(sm_count > 0 ? sm_count : 148) * 2 * kSearchWarps;
+    // Measured on a B200 (the autotuner's ladder, three key sets per size, seven parameter sets,
+    // build ms): bucket pipelines of 8 warps take 0.94 to 1.01 of the time of 4 warps up to 256
+    // partitions (one partition per SM at most, or two) and 0.97 to 1.4 above; 4 warps win up to
+    // 2048 partitions (0.59-0.93 against 0.72-1.34 ms on one warp) and are level with one warp
+    // per partition at 4096 (0.90 to 1.14 of each other), so the line lies between.
     SearchShape sh;
     sh.group = 1;
-    if ((uint64_t)partitions * 8 <= wave && partitions <= 256) sh = SearchShape{8, true};
-    else if ((uint64_t)partitions * 4 <= wave && partitions <= 512) sh = SearchShape{4, true};
-    else if ((uint64_t)partitions * 2 <= wave && partitions <= 1024) sh = SearchShape{2, true};
+    const uint64_t sms = sm_count > 0 ? sm_count : 148;
+    if (partitions <= 256 && partitions <= 2 * sms) sh = SearchShape{8, true};
+    else if (partitions <= 21 * sms) sh = SearchShape{4, true};  // 3108 on 148 SMs
     return sh;
 }
 
