@@ -14,13 +14,18 @@
 // phobic_encode's for the same arrays.
 //
 //   k_colmax     per column (an interleaved column of `partitions` pilots, or the
-//                one mono column of all pilots): largest value
-//   k_codemax    largest partition-offset code (zig-zag difference to i * P, or
-//                the offset itself)
-//   k_pack       one thread per output word of every column; writes the headers
+//                one mono column of all pilots): largest value; and the largest
+//                partition-offset code (zig-zag difference to i * P, or the offset
+//                itself)
+//   k_table      widths and byte offsets of all columns (one CTA)
+//   k_pack       one thread per output word of every column; writes the headers,
+//                unless the output does not fit (the host then packs into a stage)
 //
 // A column's words depend only on its values and width, so all columns are
-// written by one launch from a table of (values, count, width, byte offset).
+// written by one launch from the table.  The widths are known on the device only: with
+// the table made there, the call waits for the device once, at its end.  At 10^8 keys
+// (57 MB of pilots) the call took 132 us with the table made on the host between the
+// maxima and the packing (three copies, a wait, one copy), and takes 97 us.
 #include <algorithm>
 #include <cstring>
 #include <vector>
@@ -33,6 +38,7 @@ namespace phobicb200 {
 namespace {
 
 constexpr int kEncThreads = 256;
+constexpr int kMaxLoads = 8;  // loads in flight per thread of k_colmax
 
 // One compact vector of the output.
 struct EncColumn {
@@ -54,36 +60,97 @@ __device__ __forceinline__ uint64_t offset_code(const uint32_t *off, uint64_t i,
 
 __device__ __forceinline__ uint64_t words_for(uint64_t bits) { return (bits + 63) / 64; }
 
-// Largest value of column blockIdx.y, per CTA chunk, into maxes[y] (atomicMax).
-__global__ void __launch_bounds__(kEncThreads) k_colmax(const uint32_t *pilots, uint64_t per_col, uint32_t *maxes) {
-    const uint32_t *v = pilots + (uint64_t)blockIdx.y * per_col;
+// Largest value of column blockIdx.x, per CTA chunk, into maxes[x] (atomicMax); the last
+// blockIdx.x: largest partition-offset code into *code_max.
+__global__ void __launch_bounds__(kEncThreads) k_colmax(const uint32_t *pilots, uint64_t per_col, uint32_t cols,
+                                                        uint32_t *maxes, const uint32_t *off, uint64_t noff,
+                                                        uint32_t psize, int diff, unsigned long long *code_max) {
+    const uint64_t first = (uint64_t)blockIdx.y * blockDim.x + threadIdx.x, step = (uint64_t)gridDim.y * blockDim.x;
+    if (blockIdx.x == cols) {
+        unsigned long long m = 0;
+        for (uint64_t i = first; i < noff; i += step) m = max(m, (unsigned long long)offset_code(off, i, psize, diff != 0));
+        for (int d = 16; d; d >>= 1) m = max(m, __shfl_xor_sync(kFullMask, m, d));
+        if ((threadIdx.x & 31) == 0 && m) atomicMax(code_max, m);
+        return;
+    }
+    const uint32_t *v = pilots + (uint64_t)blockIdx.x * per_col;
     uint32_t m = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < per_col; i += (uint64_t)gridDim.x * blockDim.x)
-        m = max(m, __ldg(v + i));
+    for (uint64_t i = first; i < per_col; i += kMaxLoads * step) {  // the loads of a round in flight together
+        uint32_t x[kMaxLoads];
+#pragma unroll
+        for (int j = 0; j < kMaxLoads; j++) x[j] = i + j * step < per_col ? __ldg(v + i + j * step) : 0u;
+#pragma unroll
+        for (int j = 0; j < kMaxLoads; j++) m = max(m, x[j]);
+    }
     m = __reduce_max_sync(kFullMask, m);
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(&maxes[blockIdx.y], m);
+    if ((threadIdx.x & 31) == 0 && m) atomicMax(&maxes[blockIdx.x], m);
 }
 
-__global__ void __launch_bounds__(kEncThreads) k_codemax(const uint32_t *off, uint64_t count, uint32_t psize, int diff,
-                                                         unsigned long long *mx) {
-    unsigned long long m = 0;
-    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < count; i += (uint64_t)gridDim.x * blockDim.x)
-        m = max(m, (unsigned long long)offset_code(off, i, psize, diff != 0));
-    for (int d = 16; d; d >>= 1) m = max(m, __shfl_xor_sync(kFullMask, m, d));
-    if ((threadIdx.x & 31) == 0 && m) atomicMax(mx, m);
+// Bytes of a compact vector of n values of width w: size, width, mask, count, words.
+__host__ __device__ __forceinline__ uint64_t vector_bytes(uint64_t n, uint32_t w) { return 32 + 8 * ((n * w + 63) / 64 + 1); }
+
+// The column table in visit order (pilot columns, then the offsets) from the maxima; info[0] = the
+// size of the output, info[1] = keys.  One CTA: each thread takes the columns tid + 256 k, a chunk
+// of 256 columns at a time.
+__global__ void __launch_bounds__(kEncThreads) k_table(const uint32_t *maxes, const unsigned long long *code_max,
+                                                       const uint32_t *pilots, uint64_t per_col, uint32_t cols,
+                                                       const uint32_t *off, uint64_t noff, EncColumn *table,
+                                                       unsigned long long *info) {
+    __shared__ unsigned long long sums[kEncThreads / 32];
+    const uint32_t tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+    unsigned long long at = 0;
+    for (uint32_t c0 = 0; c0 <= cols; c0 += kEncThreads) {
+        const uint32_t c = c0 + tid;
+        EncColumn e{nullptr, 0, 0, 0, 0};
+        unsigned long long bytes = 0;
+        if (c <= cols) {
+            const unsigned long long m = c < cols ? maxes[c] : *code_max;
+            e.vals = c < cols ? pilots + (uint64_t)c * per_col : nullptr;
+            e.n = c < cols ? per_col : noff;
+            e.width = m ? 64 - __clzll((long long)m) : 1;
+            bytes = vector_bytes(e.n, e.width);
+        }
+        unsigned long long incl = bytes;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned long long t = __shfl_up_sync(kFullMask, incl, d);
+            if (lane >= (uint32_t)d) incl += t;
+        }
+        if (lane == 31) sums[warp] = incl;
+        __syncthreads();
+        unsigned long long total = 0;
+        for (uint32_t v = 0; v < kEncThreads / 32; v++) {
+            if (v < warp) incl += sums[v];
+            total += sums[v];
+        }
+        if (c <= cols) {
+            e.out = at + incl - bytes;
+            table[c] = e;
+        }
+        at += total;
+        __syncthreads();
+    }
+    if (tid == 0) {
+        info[0] = at;
+        info[1] = off[noff - 1];
+    }
 }
 
 // Word t of column blockIdx.x / per_col (t = index among the vector's words, the
 // column's CTAs striding over them; the header's four u64 are written by t = 0).
-// Words past ceil(n w / 64) are zero.
+// Words past ceil(n w / 64) are zero.  Nothing is written when the output exceeds `room`.
 __global__ void __launch_bounds__(kEncThreads) k_pack(const EncColumn *cols, uint32_t per_col, const uint32_t *off,
-                                                      uint32_t psize, int diff, uint8_t *out) {
+                                                      uint32_t psize, int diff, uint8_t *out,
+                                                      const unsigned long long *info, uint64_t room) {
+    if (info[0] > room) return;
     const EncColumn c = cols[blockIdx.x / per_col];
     const uint64_t chunk = blockIdx.x % per_col;
-    const uint64_t w = c.width;
-    const uint64_t words = words_for(c.n * w) + 1;
+    const uint32_t w = c.width;
+    const uint64_t bits_used = c.n * w;
+    const uint64_t words = words_for(bits_used) + 1;
     uint64_t *hdr = reinterpret_cast<uint64_t *>(out + c.out);
     uint64_t *bits = hdr + 4;
+    const bool narrow = bits_used + 64 < 0xFFFFFFFFull;  // bit positions fit 32 bits: a 64-bit division costs four times as much
     for (uint64_t t = chunk * blockDim.x + threadIdx.x; t < words; t += (uint64_t)per_col * blockDim.x) {
         if (t == 0) {
             hdr[0] = c.n;
@@ -91,25 +158,20 @@ __global__ void __launch_bounds__(kEncThreads) k_pack(const EncColumn *cols, uin
             hdr[2] = w == 64 ? ~0ull : (1ull << w) - 1;
             hdr[3] = words;
         }
-        const uint64_t lo = 64 * t, hi = lo + 64;  // bits of this word
+        const uint64_t lo = 64 * t;  // first bit of this word
         uint64_t word = 0;
-        if (lo < c.n * w) {
-            const uint64_t i0 = lo / w;
-            uint64_t i1 = (hi - 1) / w;
-            if (i1 >= c.n) i1 = c.n - 1;
-            for (uint64_t i = i0; i <= i1; i++) {
+        if (lo < bits_used) {
+            uint64_t i = narrow ? (uint32_t)lo / w : lo / w;
+            // Value i may begin before the word; the following ones begin inside it.
+            int32_t pos = (int32_t)(i * w - lo);
+            for (; pos < 64 && i < c.n; i++, pos += (int32_t)w) {
                 const uint64_t v = c.vals ? (uint64_t)__ldg(c.vals + i) : offset_code(off, i, psize, diff != 0);
-                const uint64_t pos = i * w;
-                word |= pos >= lo ? v << (pos - lo) : v >> (lo - pos);
+                word |= pos >= 0 ? v << pos : v >> -pos;
             }
         }
         bits[t] = word;
     }
 }
-
-uint32_t width_of(uint64_t max_value) { return max_value ? 64 - __builtin_clzll(max_value) : 1; }
-uint64_t host_words(uint64_t bits) { return (bits + 63) / 64; }
-uint64_t vector_bytes(uint64_t n, uint32_t w) { return 32 + 8 * (host_words(n * w) + 1); }
 
 }  // namespace
 
@@ -127,11 +189,12 @@ phobic_status run_encode_gpu(Worker &w, DeviceArena &out_arena, int pilot_encode
     const bool mono = pilot_encoder == 3;
     const uint32_t cols = mono ? 1u : (uint32_t)B;
     PHB_TRY(cudaSetDevice(w.device), "cudaSetDevice");
-    PHB_TRY(w.pinned.reserve(4096 + 4 * (size_t)cols + sizeof(EncColumn) * (cols + 1)), "pinned");
+    PHB_TRY(w.pinned.reserve(4096), "pinned");
     cudaStream_t s = w.stream;
 
-    // Inputs on the device, the maxima, the column table.
-    const size_t need = align256(4 * npil) + align256(4 * noff) + align256(4 * (size_t)cols) + align256(8) +
+    // Inputs on the device; the maxima and {size, keys}; the column table.
+    const size_t max_bytes = align256(8 + 4 * (size_t)cols);
+    const size_t need = align256(4 * npil) + align256(4 * noff) + max_bytes + align256(16) +
                         align256(sizeof(EncColumn) * (cols + 1)) + 4096;
     w.arena.reset();
     PHB_TRY(w.arena.reserve(need), "device arena");
@@ -143,75 +206,53 @@ phobic_status run_encode_gpu(Worker &w, DeviceArena &out_arena, int pilot_encode
         PHB_TRY(cudaMemcpyAsync(b, built->partition_offsets, 4 * noff, cudaMemcpyHostToDevice, s), "H2D offsets");
         d_pil = a, d_off = b;
     }
-    uint32_t *d_max = static_cast<uint32_t *>(w.arena.take(4 * (size_t)cols));
-    unsigned long long *d_cmax = static_cast<unsigned long long *>(w.arena.take(8));
+    unsigned long long *d_cmax = static_cast<unsigned long long *>(w.arena.take(max_bytes));
+    uint32_t *d_max = reinterpret_cast<uint32_t *>(d_cmax + 1);
+    unsigned long long *d_info = static_cast<unsigned long long *>(w.arena.take(16));
     EncColumn *d_cols = static_cast<EncColumn *>(w.arena.take(sizeof(EncColumn) * (cols + 1)));
-    PHB_TRY(cudaMemsetAsync(d_max, 0, 4 * (size_t)cols, s), "memset");
-    PHB_TRY(cudaMemsetAsync(d_cmax, 0, 8, s), "memset");
+    PHB_TRY(cudaMemsetAsync(d_cmax, 0, max_bytes, s), "memset");
     const uint64_t per_col = mono ? npil : P;
-    if (per_col) {
-        const uint32_t gx = (uint32_t)std::min<uint64_t>((per_col + kEncThreads * 8 - 1) / (kEncThreads * 8),
-                                                         mono ? (uint64_t)w.sm_count * 8 : 64);
-        k_colmax<<<dim3(gx, cols), kEncThreads, 0, s>>>(d_pil, per_col, d_max);
-        PHB_TRY(cudaGetLastError(), "k_colmax");
-    }
     const uint32_t psize = params->partition_size;
     const int diff = offset_encoder == 0;
-    k_codemax<<<(uint32_t)std::min<uint64_t>((noff + kEncThreads - 1) / kEncThreads, 1024), kEncThreads, 0, s>>>(
-        d_off, noff, psize, diff, d_cmax);
-    PHB_TRY(cudaGetLastError(), "k_codemax");
-    uint8_t *hp = static_cast<uint8_t *>(w.pinned.data());
-    uint32_t *h_max = reinterpret_cast<uint32_t *>(hp + 64);
-    unsigned long long *h_cmax = reinterpret_cast<unsigned long long *>(hp);
-    uint32_t *h_n = reinterpret_cast<uint32_t *>(hp + 8);
-    PHB_TRY(cudaMemcpyAsync(h_max, d_max, 4 * (size_t)cols, cudaMemcpyDeviceToHost, s), "D2H maxima");
-    PHB_TRY(cudaMemcpyAsync(h_cmax, d_cmax, 8, cudaMemcpyDeviceToHost, s), "D2H maxima");
-    PHB_TRY(cudaMemcpyAsync(h_n, d_off + P, 4, cudaMemcpyDeviceToHost, s), "D2H n");
+    const uint32_t gy = (uint32_t)std::max<uint64_t>(
+        1, std::min<uint64_t>((std::max(per_col, noff) + kEncThreads * kMaxLoads - 1) / (kEncThreads * kMaxLoads),
+                              mono ? (uint64_t)w.sm_count * 8 : 64));
+    k_colmax<<<dim3(cols + 1, gy), kEncThreads, 0, s>>>(d_pil, per_col, cols, d_max, d_off, noff, psize, diff, d_cmax);
+    PHB_TRY(cudaGetLastError(), "k_colmax");
+    k_table<<<1, kEncThreads, 0, s>>>(d_max, d_cmax, d_pil, per_col, cols, d_off, noff, d_cols, d_info);
+    PHB_TRY(cudaGetLastError(), "k_table");
+    // The widths are not known here: CTAs for columns of up to 32-bit values (they stride over more).
+    const uint64_t max_words = (std::max(per_col, noff) + 1) / 2 + 2;
+    const uint64_t per = std::min<uint64_t>((max_words + kEncThreads - 1) / kEncThreads,
+                                            std::max<uint64_t>(1, (uint64_t)w.sm_count * 16 / (cols + 1)));
+    auto pack = [&](uint8_t *to, uint64_t room) {
+        k_pack<<<(uint32_t)(per * (cols + 1)), kEncThreads, 0, s>>>(d_cols, (uint32_t)per, d_off, psize, diff, to, d_info,
+                                                                    room);
+        return cudaGetLastError();
+    };
+    // The kernel stores 8-byte words: only a device destination that is 8-byte aligned and large
+    // enough is written directly.
+    const bool direct = out && out_on_device && !(reinterpret_cast<uintptr_t>(out) & 7);
+    if (direct) PHB_TRY(pack(out, cap), "k_pack");
+    unsigned long long *h_info = static_cast<unsigned long long *>(w.pinned.data());
+    PHB_TRY(cudaMemcpyAsync(h_info, d_info, 16, cudaMemcpyDeviceToHost, s), "D2H size");
     PHB_TRY(cudaEventRecord(w.ev[7], s), "event");
     phobic_status st = wait_event(w.ev[7], w.timeout_ms, err);
     if (st != PHOBIC_OK) return st;
-
-    // Column table and sizes (host), in visit order: pilot columns, then the offsets.
-    EncColumn *h_cols = reinterpret_cast<EncColumn *>(hp + 64 + align256(4 * (size_t)cols));
-    uint64_t total = 0;
-    for (uint32_t j = 0; j < cols; j++) {
-        const uint32_t wd = width_of(h_max[j]);
-        h_cols[j] = EncColumn{d_pil + (uint64_t)j * per_col, per_col, total, wd, 0};
-        total += vector_bytes(per_col, wd);
-    }
-    const uint32_t wo = width_of(*h_cmax);
-    h_cols[cols] = EncColumn{nullptr, noff, total, wo, 0};
-    total += vector_bytes(noff, wo);
+    const uint64_t total = h_info[0], n = h_info[1];
     *size = total;
-    if (bits_per_key) {
-        // getBitsPerKey (mphf.hpp:88-91): encoder bits (8 per serialised byte), fulcrums and partition count.
-        const uint64_t n = *h_n;
-        *bits_per_key = n ? (double)(float(total * 8 + 32 * (uint64_t)kFulcrums + 32 * P) / float(n)) : 0.0;
-    }
-    if (!out) return PHOBIC_OK;
+    // getBitsPerKey (mphf.hpp:88-91): encoder bits (8 per serialised byte), fulcrums and partition count.
+    if (bits_per_key) *bits_per_key = n ? (double)(float(total * 8 + 32 * (uint64_t)kFulcrums + 32 * P) / float(n)) : 0.0;
+    if (!out || (direct && total <= cap)) return PHOBIC_OK;
 
-    // The kernel stores 8-byte words: a device destination that is too small or not
-    // 8-byte aligned is written through the staging buffer.
-    uint8_t *d_out = out;
-    if (!out_on_device || cap < total || (reinterpret_cast<uintptr_t>(out) & 7)) {
-        PHB_TRY(out_arena.reserve(total), "device output");
-        out_arena.reset();
-        d_out = static_cast<uint8_t *>(out_arena.take(total));
-    }
-    PHB_TRY(cudaMemcpyAsync(d_cols, h_cols, sizeof(EncColumn) * (cols + 1), cudaMemcpyHostToDevice, s), "H2D table");
-    uint64_t max_words = 0;
-    for (uint32_t j = 0; j <= cols; j++) max_words = std::max(max_words, host_words(h_cols[j].n * h_cols[j].width) + 1);
-    const uint64_t per = std::min<uint64_t>((max_words + kEncThreads - 1) / kEncThreads,
-                                            std::max<uint64_t>(1, (uint64_t)w.sm_count * 16 / (cols + 1)));
-    k_pack<<<(uint32_t)(per * (cols + 1)), kEncThreads, 0, s>>>(d_cols, (uint32_t)per, d_off, psize, diff, d_out);
-    PHB_TRY(cudaGetLastError(), "k_pack");
-    if (d_out != out) {
-        const size_t ncopy = std::min<size_t>(cap, total);
-        if (ncopy)
-            PHB_TRY(cudaMemcpyAsync(out, d_out, ncopy, out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost,
-                                    s),
-                    "copy out");
-    }
+    PHB_TRY(out_arena.reserve(total), "device output");
+    out_arena.reset();
+    uint8_t *d_out = static_cast<uint8_t *>(out_arena.take(total));
+    PHB_TRY(pack(d_out, total), "k_pack");
+    const size_t ncopy = std::min<size_t>(cap, total);
+    if (ncopy)
+        PHB_TRY(cudaMemcpyAsync(out, d_out, ncopy, out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s),
+                "copy out");
     PHB_TRY(cudaEventRecord(w.ev[7], s), "event");
     return wait_event(w.ev[7], w.timeout_ms, err);
 }

@@ -29,12 +29,11 @@ def test_bucket_order_matches_oracle(phobic, lam, P, buckets):
 
 
 @pytest.mark.parametrize("group,pipe", [(1, 0), (2, 1), (4, 1), (8, 1), (4, 0)])
-@pytest.mark.parametrize("P", [31, 1024, 3072])
+@pytest.mark.parametrize("P", [1024, 2048, 3072])
 def test_round_edges_match_oracle(phobic, P, group, pipe):
-    """Partitions on both sides of 32, 1024 and 3072 slots: the edges of the offset search's words
-    and rounds, and of the pipeline's one-to-three-round and general searches."""
+    """Partitions on both sides of 1024, 2048 and 3072 slots: the edges of the offset search's
+    rounds, and of the pipeline's one-, two- and three-round and general searches."""
     cfg = phobic.MPHFconfig(5.0, P)
-    cfg.params.max_partition_size = 2 * P + 32
     keys = keygen.splitmix64(7000 + P, 40 * P + 3)
     want = O.build(O.hash_keys(keys, "u64"), P, cfg.bucketCountPerPartition, cfg.getFulcs())
     assert want["status"] == 0
