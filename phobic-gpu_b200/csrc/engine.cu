@@ -795,7 +795,7 @@ phobic_status run_query(Worker &w, const phobic_keys *keys, const phobic_params 
     const uint64_t n = keys->n;
     const uint32_t B = params->buckets;
     PHB_TRY(cudaSetDevice(w.device), "cudaSetDevice");
-    PHB_TRY(w.pinned.reserve(4096), "pinned");
+    PHB_TRY(w.pinned.reserve(256 + 4 * kFulcrums), "pinned");
     unsigned long long *hword = static_cast<unsigned long long *>(w.pinned.data());
     uint64_t bytes = 8192 + align256(4 * kFulcrums) + align256(8) + align256(4 * (size_t)B * partitions) +
                      align256(4 * ((size_t)partitions + 1)) + align256(4 * n) + align256(4 * ((n + 31) / 32 + 1)) +
@@ -821,9 +821,11 @@ phobic_status run_query(Worker &w, const phobic_keys *keys, const phobic_params 
         }
     }
     uint32_t *d_fulcs = static_cast<uint32_t *>(w.arena.take(4 * kFulcrums));
-    PHB_TRY(cudaMemcpyAsync(d_fulcs, params->fulcrums, 4 * kFulcrums, cudaMemcpyHostToDevice, s), "H2D fulcrums");
+    char *fulcs = static_cast<char *>(w.pinned.data()) + 256;  // free: every call waits for its work
+    std::memcpy(fulcs, params->fulcrums, 4 * kFulcrums);
+    PHB_TRY(cudaMemcpyAsync(d_fulcs, fulcs, 4 * kFulcrums, cudaMemcpyHostToDevice, s), "H2D fulcrums");
     unsigned long long *d_bad = static_cast<unsigned long long *>(w.arena.take(8));
-    PHB_TRY(cudaMemsetAsync(d_bad, 0, 8, s), "memset");
+    if (bad) PHB_TRY(cudaMemsetAsync(d_bad, 0, 8, s), "memset");
     const uint32_t *d_pil = built->pilots, *d_off = built->partition_offsets;
     if (!built->on_device) {
         uint32_t *a = static_cast<uint32_t *>(w.arena.take(4 * (size_t)B * partitions));
@@ -834,10 +836,13 @@ phobic_status run_query(Worker &w, const phobic_keys *keys, const phobic_params 
             return st;
         d_pil = a, d_off = b;
     }
-    PHB_TRY(cudaMemcpyAsync(hword, d_off + partitions, 4, cudaMemcpyDeviceToHost, s), "D2H n");
-    PHB_TRY(cudaEventRecord(w.ev[7], s), "event");
-    if ((st = wait_event(w.ev[7], w.timeout_ms, err)) != PHOBIC_OK) return st;
-    const uint32_t n_built = (uint32_t)(*hword & 0xFFFFFFFFull);
+    uint32_t n_built = 0;  // only the bijection check asks for it
+    if (bad) {
+        PHB_TRY(cudaMemcpyAsync(hword, d_off + partitions, 4, cudaMemcpyDeviceToHost, s), "D2H n");
+        PHB_TRY(cudaEventRecord(w.ev[7], s), "event");
+        if ((st = wait_event(w.ev[7], w.timeout_ms, err)) != PHOBIC_OK) return st;
+        n_built = (uint32_t)(*hword & 0xFFFFFFFFull);
+    }
     uint32_t *d_pos = nullptr;
     if (positions) d_pos = keys->on_device ? positions : static_cast<uint32_t *>(w.arena.take(4 * n));
     uint32_t *d_seen = nullptr;
