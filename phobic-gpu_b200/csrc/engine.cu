@@ -397,9 +397,9 @@ uint64_t sets_arena_bytes(const phobic_keys *sets, uint32_t nsets, const phobic_
         if (!results || !results[s].on_device) t += align256(4 * B * m) + align256(4 * (m + 1));
     }
     t += align256(4 * kFulcrums) + align256(sizeof(SetDesc) * nsets) + 2 * align256(8 * (nsets + 1)) +
-         align256(8 * nsets) + align256(64);
+         align256(8 * nsets);
     const uint64_t MS = M * plan_map(N, M, 0).stride;  // count matrix entries
-    t += align256(4 * MS) + align256(4 * (MS + 1)) + align256(8 * ((MS + kScanTile - 1) / kScanTile) + 8);
+    t += align256(4 * MS) + align256(4 * (MS + 1)) + align256(64 + 8 * ((MS + kScanTile - 1) / kScanTile) + 8);
     if (nsets && sets[0].kind == PHOBIC_KEYS_STRINGS) t += align256(16 * N);
     // lowers, bucket ids, partition records (also the search's scratch), cursors
     t += align256(8 * N) + align256(2 * N) + align256(16 * N) + align256(4 * M) + align256(4 * kMaxBins);
@@ -455,8 +455,8 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
     PHB_TRY(cudaSetDevice(w.device), "cudaSetDevice");
 
     // Host-side set table (pinned): SetDesc[nsets] | key_base[nsets+1] | part_base[nsets+1] |
-    // fulcrums | err[nsets].  Everything before err goes up in one copy to the same layout on
-    // the device.
+    // fulcrums | err[nsets].  It goes up in one copy to the same layout on the device, the error
+    // words as "no error"; they come back to their place at the end.
     const size_t tab_desc = align256(sizeof(SetDesc) * nsets), tab_kb = align256(8 * (nsets + 1)),
                  tab_pb = align256(8 * (nsets + 1)), tab_fulcs = align256(4 * kFulcrums), tab_err = align256(8 * nsets);
     const size_t tab_in = tab_desc + tab_kb + tab_pb + tab_fulcs;
@@ -468,6 +468,7 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
     std::memcpy(tab + tab_desc + tab_kb + tab_pb, params->fulcrums, 4 * kFulcrums);
     w.pending_err = reinterpret_cast<unsigned long long *>(tab + tab_in);
     w.pending_sets = nsets;
+    std::fill_n(w.pending_err, nsets, kNoError);
 
     // Host results: pinned destinations are copied to directly, pageable ones through the
     // worker's pinned stage (sized here, before any launch, since growing it reallocates).
@@ -541,18 +542,20 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
     }
     hkb[nsets] = kb;
     hpb[nsets] = pb;
-    char *d_tab = static_cast<char *>(take(tab_in));
+    char *d_tab = static_cast<char *>(take(tab_in + tab_err));
     SetDesc *d_desc = reinterpret_cast<SetDesc *>(d_tab);
     uint64_t *d_kb = reinterpret_cast<uint64_t *>(d_tab + tab_desc);
     uint32_t *d_pb = reinterpret_cast<uint32_t *>(d_tab + tab_desc + tab_kb);
     uint32_t *d_fulcs = reinterpret_cast<uint32_t *>(d_tab + tab_desc + tab_kb + tab_pb);
-    unsigned long long *d_err = static_cast<unsigned long long *>(take(8 * nsets));
-    uint32_t *d_queue = static_cast<uint32_t *>(take(64));
+    unsigned long long *d_err = reinterpret_cast<unsigned long long *>(d_tab + tab_in);
     const uint64_t MS = M * plan.stride;  // count matrix entries
     uint32_t *d_count = static_cast<uint32_t *>(take(4 * MS));
     uint32_t *d_G = static_cast<uint32_t *>(take(4 * (MS + 1)));
     const uint32_t tiles = (uint32_t)((MS + kScanTile - 1) / kScanTile);
-    unsigned long long *d_tiles = static_cast<unsigned long long *>(take(8 * (size_t)tiles + 8));
+    // What a build finds at zero, side by side: the search's queue, the scan's tiles and tile counter.
+    const size_t zero_bytes = 64 + 8 * (size_t)tiles + 8;
+    uint32_t *d_queue = static_cast<uint32_t *>(take(zero_bytes));
+    unsigned long long *d_tiles = reinterpret_cast<unsigned long long *>(d_queue + 16);
     uint4 *d_mapped = kind == PHOBIC_KEYS_STRINGS ? static_cast<uint4 *>(take(16 * N)) : nullptr;
     uint2 *d_lowers = static_cast<uint2 *>(take(8 * N));
     uint16_t *d_bkt = static_cast<uint16_t *>(take(2 * N));
@@ -566,7 +569,7 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
         if (err) *err = "arena sizing error";
         return PHOBIC_ERR_OOM;
     }
-    PHB_TRY(cudaMemcpyAsync(d_tab, tab, tab_in, cudaMemcpyHostToDevice, s), "H2D set table and fulcrums");
+    PHB_TRY(cudaMemcpyAsync(d_tab, tab, tab_in + tab_err, cudaMemcpyHostToDevice, s), "H2D set table and fulcrums");
     uint64_t kc_index = 0, kc_mask = 0;
     const bool key_change = nsets == 1 && take_key_change(N, kind, &kc_index, &kc_mask);
     const uint32_t wshift = part_wshift(M);
@@ -585,10 +588,9 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
         auto record = [&](cudaEvent_t e) {
             return capture ? cudaEventRecordWithFlags(e, s, cudaEventRecordExternal) : cudaEventRecord(e, s);
         };
-        PHB_TRY(cudaMemsetAsync(d_err, 0xFF, 8 * nsets, s), "memset");
-        PHB_TRY(cudaMemsetAsync(d_queue, 0, 64, s), "memset");
-        PHB_TRY(cudaMemsetAsync(d_count, 0, 4 * MS, s), "memset");
-        PHB_TRY(cudaMemsetAsync(d_tiles, 0, 8 * (size_t)tiles + 8, s), "memset");
+        PHB_TRY(cudaMemsetAsync(d_queue, 0, zero_bytes, s), "memset");
+        // 32-bit chunk counters write their whole columns.
+        if (MS && !(plan.chunked && !plan.narrow)) PHB_TRY(cudaMemsetAsync(d_count, 0, 4 * MS, s), "memset");
         if (M == 0) PHB_TRY(cudaMemsetAsync(d_G, 0, 4, s), "memset");
         PHB_TRY(record(w.ev[1]), "event");
         // K1, scan, two partition passes, bucket order, search; none when there are no keys.

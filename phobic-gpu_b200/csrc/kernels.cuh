@@ -24,7 +24,9 @@ constexpr int kMapThreads = 256;
 // exclusive scan gives each chunk its own slot range inside every partition.
 constexpr int kChunkThreads = 1024;
 constexpr uint32_t kChunkCtas = 148;                 // one CTA per SM of a B200
-constexpr uint64_t kChunkMinKeys = 16384;            // smallest chunk worth a CTA
+// Smallest chunk worth a CTA, two keys a thread: against 16,384 keys the counting of 700,001 strings
+// takes 25 us, not 60, of 10^6 u64 keys 11, not 15.
+constexpr uint64_t kChunkMinKeys = 2048;
 constexpr uint32_t kChunkMaxPartitions = 52 * 1024;  // 32-bit shared-memory counters per CTA
 // Counting only (K1): above kChunkMaxPartitions the counters are packed two to a
 // 32-bit word.  A 16-bit counter that wraps is caught from the atomic's return value
@@ -212,9 +214,9 @@ struct SearchShape {
 };
 cudaError_t launch_search(const SearchArgs &a, int sm_count, cudaStream_t st, SearchShape shape = SearchShape{});
 // Default shape when the autotuner's table has no line for a build, fitted to the B200's
-// measurements: bucket pipelines of 8 warps up to 256 partitions, of 4 up to about 3100, else
-// one warp per partition.
-SearchShape search_shape_for(uint32_t partitions, int sm_count);
+// measurements: bucket pipelines of 8 warps up to 256 partitions, of 4 up to about 2700 (4400
+// where many pilot counters fail), else one warp per partition.
+SearchShape search_shape_for(uint32_t partitions, uint32_t partition_size, uint32_t buckets, int sm_count);
 size_t search_group_smem(uint32_t buckets, uint32_t cap, int W);
 // First failed bounds check of each kernel file in the checked build (source line, 0 =
 // none; always 0 in the normal build); reset clears it.

@@ -1085,23 +1085,25 @@ static cudaError_t launch_group(const SearchArgs &a, int sm_count, cudaStream_t 
     return cudaGetLastError();
 }
 
-SearchShape search_shape_for(uint32_t partitions, int sm_count) {
+SearchShape search_shape_for(uint32_t partitions, uint32_t partition_size, uint32_t buckets, int sm_count) {
     // Measured on a B200 (the autotuner's ladder, three key sets per size, seven parameter sets,
-    // build ms): bucket pipelines of 8 warps take 0.94 to 1.01 of the time of 4 warps up to 256
-    // partitions (one partition per SM at most, or two) and 0.97 to 1.4 above; 4 warps win up to
-    // 2048 partitions (0.59-0.93 against 0.72-1.34 ms on one warp) and are level with one warp
-    // per partition at 4096 (0.90 to 1.14 of each other), so the line lies between.
+    // build ms): bucket pipelines of 8 warps take 0.89 to 0.99 of the time of 4 warps up to 256
+    // partitions (at most two per SM) and 0.96 to 1.4 above; 4 warps win up to 2048 partitions
+    // (0.54-1.16 against 0.63-1.60 ms on one warp).  At 4096 they are level with one warp per
+    // partition where few pilot counters fail (average bucket of 6 keys and less: 0.97-1.18 against
+    // 0.83-1.02 ms) and still ahead where many do (7 and more: 1.30-2.04 against 1.33-2.40 ms).
     SearchShape sh;
     sh.group = 1;
     const uint64_t sms = sm_count > 0 ? sm_count : 148;
+    const bool retries = (uint64_t)partition_size * 2 >= (uint64_t)buckets * 13;
     if (partitions <= 256 && partitions <= 2 * sms) sh = SearchShape{8, true};
-    else if (partitions <= 21 * sms) sh = SearchShape{4, true};  // 3108 on 148 SMs
+    else if (partitions <= (retries ? 30 : 18) * sms) sh = SearchShape{4, true};  // 4440 or 2664 on 148 SMs
     return sh;
 }
 
 cudaError_t launch_search(const SearchArgs &a, int sm_count, cudaStream_t st, SearchShape shape) {
     if (a.M == 0) return cudaSuccess;
-    if (shape.group == 0) shape = search_shape_for(a.M, sm_count);
+    if (shape.group == 0) shape = search_shape_for(a.M, a.partition_size, a.buckets, sm_count);
     const int group = shape.group;
     const bool pipeline = shape.pipeline;
     if (group == 2 || group == 4 || group == 8) {
