@@ -579,7 +579,8 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
     ScanArgs sa{d_count, d_G, nullptr, (uint32_t)MS, d_tiles, reinterpret_cast<uint32_t *>(d_tiles + tiles), nsets,
                 d_err, 0, d_pcur, d_bincur, plan.stride, wshift};
     PartArgs pa{d_inter, d_bincur, d_pcur, wshift, (uint32_t)((M + (1ull << wshift) - 1) >> wshift), (uint32_t)M};
-    SearchArgs qa{d_desc, d_pb, nsets, (uint32_t)M, d_G, plan.stride, d_lowers, d_bkt, d_sorted, d_dbg_sizes, B, cap,
+    const bool small = nsets == 1 && !debug && !key_change && gather_fits(kind, N, M, B, cap);
+    SearchArgs qa{d_desc, d_pb, nsets, (uint32_t)M, d_G, small ? 1u : plan.stride, d_lowers, d_bkt, d_sorted, d_dbg_sizes, B, cap,
                   k_max, d_queue, d_err, d_pcur, P};
 
     // The device stages, from the per-build memsets to the status copy: enqueued one by one,
@@ -589,6 +590,21 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
             return capture ? cudaEventRecordWithFlags(e, s, cudaEventRecordExternal) : cudaEventRecord(e, s);
         };
         PHB_TRY(cudaMemsetAsync(d_queue, 0, zero_bytes, s), "memset");
+        if (small) {
+            PHB_TRY(record(w.ev[1]), "event");
+            {
+                StageRange r("bucket_sizes, partition_offsets, key_redistribution (K1-K3)");
+                PHB_TRY(launch_gather(kind, ma, qa, d_G, d_count, d_queue + 8, s), "gather");
+            }
+            for (int e = 2; e <= 4; e++) PHB_TRY(record(w.ev[e]), "event");
+            {
+                StageRange r("search (K4)");
+                PHB_TRY(launch_search(qa, w.sm_count, s, shape), "K4 search");
+            }
+            PHB_TRY(record(w.ev[5]), "event");
+            PHB_TRY(cudaMemcpyAsync(w.pending_err, d_err, 8 * nsets, cudaMemcpyDeviceToHost, s), "D2H status");
+            return PHOBIC_OK;
+        }
         // 32-bit chunk counters write their whole columns.
         if (MS && !(plan.chunked && !plan.narrow)) PHB_TRY(cudaMemsetAsync(d_count, 0, 4 * MS, s), "memset");
         if (M == 0) PHB_TRY(cudaMemsetAsync(d_G, 0, 4, s), "memset");
@@ -620,7 +636,7 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
         PHB_TRY(cudaMemcpyAsync(w.pending_err, d_err, 8 * nsets, cudaMemcpyDeviceToHost, s), "D2H status");
         return PHOBIC_OK;
     };
-    w.pending_kernels = N ? 6 : 0;
+    w.pending_kernels = !N ? 0 : small ? 2 : 6;
     w.pending_graph = false;
     cudaStreamCaptureStatus cap_status = cudaStreamCaptureStatusNone;
     if (w.graphs_off || debug || key_change || !N || M > kGraphMaxPartitions ||
@@ -631,7 +647,7 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
         // Everything the launches depend on: sizes, parameters, plan, shape and every buffer.
         std::vector<uint64_t> key{nsets, (uint64_t)kind, N, M, B, cap, k_max, plan.stride, plan.chunk, plan.grid,
                                   (uint64_t)plan.chunked | (uint64_t)plan.narrow << 1, wshift, tiles,
-                                  (uint64_t)shape.group, (uint64_t)shape.pipeline, (uint64_t)w.sm_count};
+                                  (uint64_t)shape.group, (uint64_t)shape.pipeline, (uint64_t)w.sm_count, (uint64_t)small};
         for (const void *p : {(const void *)d_fulcs, (const void *)d_desc, (const void *)d_kb, (const void *)d_pb,
                               (const void *)d_err, (const void *)d_queue, (const void *)d_count, (const void *)d_G,
                               (const void *)d_tiles, (const void *)d_mapped, (const void *)d_lowers,

@@ -1,6 +1,7 @@
 """The bucket order of K3c where its branches meet: bucket counts around the two-per-thread
 order (256, 512), partitions around the staged size (4096 keys), odd and tiny ones, and small
 partitions whose buckets collide on most pilot counters (the collision test at the mark)."""
+import numpy as np
 import pytest
 
 import keygen
@@ -41,3 +42,50 @@ def test_round_edges_match_oracle(phobic, P, group, pipe):
         ctx.set_tuning(search_group=group, search_pipeline=pipe)
         got = ctx.build(keys, cfg)
     assert (got.pilots == want["pilots"]).all() and (got.partition_offsets == want["offsets"]).all()
+
+
+@pytest.mark.parametrize("kind", ["u64", "bytes16", "prehashed"])
+@pytest.mark.parametrize("P,n", [(2048, 12_288), (2048, 12_289), (64, 9_472), (64, 9_473), (64, 5_001), (2500, 1),
+                                 (16_384, 12_288)])
+def test_small_builds_match_oracle(phobic, kind, P, n):
+    """Sizes on both sides of the one-launch path of small builds: 12,288 keys, 148 partitions."""
+    cfg = phobic.MPHFconfig(4.0, P)
+    if kind == "u64":
+        keys = keygen.splitmix64(50 + P, n)
+        keys4 = O.hash_keys(keys, "u64")
+    else:
+        keys = keygen.splitmix64(51 + P, 2 * n).reshape(n, 2)
+        keys4 = O.hash_keys(keys, "pairs") if kind == "bytes16" else keys.view("uint32").reshape(n, 4)
+    kid = {"u64": phobic.KEYS_U64, "bytes16": phobic.KEYS_BYTES16, "prehashed": phobic.KEYS_PREHASHED}[kind]
+    want = O.build(keys4, P, cfg.bucketCountPerPartition, cfg.getFulcs())
+    with phobic.Context(0) as ctx:
+        if want["status"] != 0:
+            with pytest.raises(phobic.PhobicError) as e:
+                ctx.build(keys, cfg, kind=kid)
+            assert e.value.status == want["status"]
+            return
+        got = ctx.build(keys, cfg, kind=kid)
+        assert got.timings["kernels"] == (2 if n <= 12_288 and got.partitions <= 148 else 6)
+    assert (got.pilots == want["pilots"]).all() and (got.partition_offsets == want["offsets"]).all()
+
+
+def test_small_builds_report_errors_like_the_oracle(phobic):
+    cfg = phobic.MPHFconfig(5.0, 2048)
+    keys = keygen.splitmix64(60, 9_000)
+    dup = keys.copy()
+    dup[7] = dup[8_000]
+    crowded = np.zeros((9_000, 4), np.uint32)  # every key in partition 0
+    crowded[:, 1:] = keygen.splitmix64(61, 2 * 9_000).view(np.uint32).reshape(9_000, 4)[:, 1:]
+    flat = crowded.copy()
+    flat[:, 0] = keygen.splitmix64(62, 9_000).astype(np.uint32)
+    flat[:, 1] = 0  # every key in bucket 0 of its partition
+    with phobic.Context(0) as ctx:
+        for k, kind, keys4 in ((dup, phobic.KEYS_U64, O.hash_keys(dup, "u64")), (crowded, phobic.KEYS_PREHASHED, crowded),
+                               (flat, phobic.KEYS_PREHASHED, flat)):
+            want = O.build(keys4, 2048, cfg.bucketCountPerPartition, cfg.getFulcs())["status"]
+            assert want != 0
+            with pytest.raises(phobic.PhobicError) as e:
+                ctx.build(k, cfg, kind=kind)
+            assert e.value.status == want
+        got = ctx.build(keys, cfg)
+        assert (got.pilots == O.build(O.hash_keys(keys, "u64"), 2048, cfg.bucketCountPerPartition, cfg.getFulcs())["pilots"]).all()
