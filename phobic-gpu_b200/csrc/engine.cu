@@ -560,7 +560,7 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
     uint2 *d_lowers = static_cast<uint2 *>(take(8 * N));
     uint16_t *d_bkt = static_cast<uint16_t *>(take(2 * N));
     uint4 *d_inter = static_cast<uint4 *>(take(16 * N));
-    uint2 *d_sorted = reinterpret_cast<uint2 *>(d_inter);  // K4 scratch, after K3 is done with d_inter
+    uint2 *d_sorted = reinterpret_cast<uint2 *>(d_inter);  // K3c, after K3b is done with d_inter
     uint32_t *d_pcur = static_cast<uint32_t *>(take(4 * M));
     uint32_t *d_bincur = static_cast<uint32_t *>(take(4 * kMaxBins));
     uint4 *d_dbg_keys = debug ? static_cast<uint4 *>(take(16 * N)) : nullptr;

@@ -7,7 +7,7 @@
 //
 // K3 replaces apply_partition_offset.comp:9-18 and redistribute_keys.comp:21-53:
 // each key's (lower1, lower2) pair and bucket id are appended to its partition.
-// The bucket order inside a partition is produced later, in shared memory, by K4.
+// The bucket order inside a partition is produced later, in shared memory, by K3c.
 //
 // Two plans (plan_map):
 //   chunked  CTA c counts (K1) and places (K3) the keys of one contiguous chunk

@@ -1,7 +1,7 @@
 // K3 as a two-pass radix partition: keys -> partition-contiguous records.
 //
 // Replaces apply_partition_offset.comp:9-18 and redistribute_keys.comp:21-53 up
-// to the order inside a partition (K4 sorts a partition by bucket in shared
+// to the order inside a partition (K3c sorts a partition by bucket in shared
 // memory).  One scattered store per key, as in a single pass with a cursor per
 // partition, leaves HBM and L2 doing 8- and 2-byte partial-sector writes; here
 // every store is part of a contiguous run:

@@ -499,7 +499,7 @@ __device__ __forceinline__ uint32_t place_large(const WarpSmem &ws, const uint2 
     return PHOBIC_ERR_SEARCH_LIMIT;
 }
 
-// The first SearchArgs words of a partition's search, by `threads` threads of which this is
+// What the search of a partition starts from, brought in by `threads` threads of which this is
 // number t: the schedule, a clear bitmap (as far as this partition reads it) and a clear
 // collision scratch.  w is the start of the group's shared memory.
 __device__ __forceinline__ void load_partition(const SearchArgs &a, uint32_t *w, const WarpSmem &ws, uint32_t base,
