@@ -152,12 +152,15 @@ __device__ __forceinline__ uint32_t window_at(const WarpSmem &ws, uint32_t addr,
 // this lane, the offsets of the last round's window that are not below ps.
 struct ScanRange {
     uint32_t ps, rounds, last_dead;
+    uint32_t dead0, dead1;  // the same for rounds 0 and 1: nothing, or last_dead where one is the last
     __device__ __forceinline__ static ScanRange make(uint32_t ps, int lane) {
         ScanRange r;
         r.ps = ps;
         r.rounds = (ps + 1023) / 1024;
         const int n = (int)ps - (int)(1024 * (r.rounds - 1)) - 32 * lane;
         r.last_dead = ~__funnelshift_lc(kFullMask, 0u, (uint32_t)max(n, 0));  // n >= 32: none
+        r.dead0 = r.rounds == 1 ? r.last_dead : 0u;
+        r.dead1 = r.rounds == 2 ? r.last_dead : 0u;
         return r;
     }
 };
@@ -184,12 +187,37 @@ __device__ __forceinline__ uint32_t round_bad(const WarpSmem &ws, const uint32_t
 }
 
 // Smallest free offset of a bucket of s <= S keys (S = 4 or 8) whose S packed slots start at the
-// shared address hs (entries past the bucket repeat a slot: OR is idempotent).  Three rounds at
-// constant offsets from each key's pair address cover 3072 offsets; larger partitions repeat
-// them.  Dead lanes read inside the padded bitmap (bitmap_pairs) and are masked.
+// shared address hs (entries past the bucket repeat a slot: OR is idempotent), in a partition of at
+// most three rounds, each at a constant offset from the keys' pair addresses.  Dead lanes read
+// inside the padded bitmap (bitmap_pairs) and are masked.
+// The masks of the rounds are held per partition: chosen in every round, with the loop over blocks
+// of rounds below for every partition, the search of 10^8 u64 keys takes 5.49 instead of 5.36 ms.
 template <int S>
 __device__ __forceinline__ uint32_t scan_small(const WarpSmem &ws, uint32_t hs, uint32_t s, const ScanRange &sr,
                                                int lane) {
+    const uint32_t lane_sa = ws.occ + 8u * lane;
+    uint32_t v[S], a[S];
+#pragma unroll
+    for (int i = 0; i < S; i += 4) {
+        const uint4 x = lds128(hs + 4 * i);
+        v[i] = x.x, v[i + 1] = x.y, v[i + 2] = x.z, v[i + 3] = x.w;
+    }
+#pragma unroll
+    for (int i = 0; i < S; i++) a[i] = lane_sa + (v[i] >> 5);
+    const bool full = s > S - 2;
+    uint32_t o;
+    if (round_result(round_bad<S, 0>(ws, a, v, full, sr.dead0), 0, &o)) return o;
+    if (sr.rounds == 1) return kNone;
+    if (round_result(round_bad<S, 1>(ws, a, v, full, sr.dead1), 1024, &o)) return o;
+    if (sr.rounds == 2) return kNone;
+    return round_result(round_bad<S, 2>(ws, a, v, full, sr.last_dead), 2048, &o) ? o : kNone;
+}
+
+// The same for a partition of more than three rounds: three at a time (scan_quads, which forms the
+// pair addresses in every round, makes the search of P = 4096 7 % slower).
+template <int S>
+__device__ __forceinline__ uint32_t scan_blocks(const WarpSmem &ws, uint32_t hs, uint32_t s, const ScanRange &sr,
+                                                int lane) {
     const uint32_t lane_sa = ws.occ + 8u * lane;
     uint32_t v[S], a[S];
 #pragma unroll
@@ -294,7 +322,8 @@ __device__ __forceinline__ uint32_t lane_key(uint32_t s, int lane) {
 // lane_key loads it.  The warp hashes 32 / S pilot counters at once (lane t * S + i holds key i
 // under counter k0 + t) into hs and tests them in counter order, so a counter that fails costs
 // no new hash.  Same result as trying k = 0, 1, 2, ... one at a time (search.comp:105-124).
-template <int S>
+// SMALL: the partition has at most three rounds.
+template <int S, bool SMALL>
 __device__ __forceinline__ uint32_t place_batched(const WarpSmem &ws, uint2 L, uint32_t s, const ScanRange &sr,
                                                   FastMod fm, uint32_t k_lim, int lane, uint32_t *pilot) {
     constexpr uint32_t G = 32 / S;
@@ -315,7 +344,8 @@ __device__ __forceinline__ uint32_t place_batched(const WarpSmem &ws, uint2 L, u
 #pragma unroll 1
         for (uint32_t u = 0; u < tries; u++) {
             uint32_t o;
-            if constexpr (S <= 8) o = scan_small<S>(ws, hs_sa + 4 * S * u, s, sr, lane);
+            if constexpr (S <= 8 && SMALL) o = scan_small<S>(ws, hs_sa + 4 * S * u, s, sr, lane);
+            else if constexpr (S <= 8) o = scan_blocks<S>(ws, hs_sa + 4 * S * u, s, sr, lane);
             else o = scan_quads(ws, hs_sa + 4 * S * u, s, sr, lane);
             if (o == kNone) continue;
             uint32_t q = unpack_slot(ws.hs[S * u + (mine ? (uint32_t)lane : 0u)]) + o;
@@ -418,7 +448,7 @@ __device__ __forceinline__ uint32_t seek_batched(const WarpSmem &ws, uint32_t *h
         const uint32_t own = hs[S * u + (mine ? (uint32_t)lane : 0u)];
         bool meet = false;
         if constexpr (NR > 0) meet = all_windows<S, NR>(ws, hs_sa + 4 * S * u, s, sr, lane, f->bad);
-        else if constexpr (S <= 8) f->o = scan_small<S>(ws, hs_sa + 4 * S * u, s, sr, lane);
+        else if constexpr (S <= 8) f->o = scan_blocks<S>(ws, hs_sa + 4 * S * u, s, sr, lane);
         else f->o = scan_quads(ws, hs_sa + 4 * S * u, s, sr, lane);
         f->h = unpack_slot(own);
         if constexpr (S == 4 && NR > 0) {
@@ -621,7 +651,7 @@ __device__ __forceinline__ void advance(const WarpSmem &ws, Cursor &c) {
 // of the class per bucket and knows the lanes' keys; the next bucket's are loaded during the search.
 // One loop for all of them takes 5.83 against 5.51 ms at 10^8 u64 keys (lambda 7), 2.46 against
 // 2.29 ms at 5*10^7 (lambda 6).
-template <int S>
+template <int S, bool SMALL = true>
 __device__ __forceinline__ uint32_t search_class(const WarpSmem &ws, const uint2 *so, const ScanRange &sr, FastMod fm,
                                                  uint32_t k_lim, uint32_t searched, int lane, Cursor &c, uint32_t *pil,
                                                  size_t pstride) {
@@ -634,7 +664,7 @@ __device__ __forceinline__ uint32_t search_class(const WarpSmem &ws, const uint2
             c.L = so[(c.sc & 0xFFFFu) + i];
         }
         uint32_t pilot = 0;
-        const uint32_t code = place_batched<S>(ws, L, s, sr, fm, k_lim, lane, &pilot);
+        const uint32_t code = place_batched<S, SMALL>(ws, L, s, sr, fm, k_lim, lane, &pilot);
         if (code != PHOBIC_OK) return code;
         if (lane == 0) pil[(size_t)b * pstride] = pilot;
     }
@@ -677,8 +707,13 @@ __device__ __forceinline__ uint32_t search_partition(const SearchArgs &a, uint32
     if (c.j < searched) c.L = so[(c.sc & 0xFFFFu) + lane_key(c.s, lane)];
     if (code == PHOBIC_OK) code = search_class<32>(ws, so, sr, fm, k_lim, searched, lane, c, pil, pstride);
     if (code == PHOBIC_OK) code = search_class<16>(ws, so, sr, fm, k_lim, searched, lane, c, pil, pstride);
-    if (code == PHOBIC_OK) code = search_class<8>(ws, so, sr, fm, k_lim, searched, lane, c, pil, pstride);
-    if (code == PHOBIC_OK) code = search_class<4>(ws, so, sr, fm, k_lim, searched, lane, c, pil, pstride);
+    if (sr.rounds <= 3) {
+        if (code == PHOBIC_OK) code = search_class<8>(ws, so, sr, fm, k_lim, searched, lane, c, pil, pstride);
+        if (code == PHOBIC_OK) code = search_class<4>(ws, so, sr, fm, k_lim, searched, lane, c, pil, pstride);
+    } else {
+        if (code == PHOBIC_OK) code = search_class<8, false>(ws, so, sr, fm, k_lim, searched, lane, c, pil, pstride);
+        if (code == PHOBIC_OK) code = search_class<4, false>(ws, so, sr, fm, k_lim, searched, lane, c, pil, pstride);
+    }
     if (code != PHOBIC_OK) return code;
     place_singles(ws, so, searched, singles, ps, fm, lane, pil, pstride);
     __syncwarp();
@@ -729,8 +764,8 @@ __device__ __forceinline__ uint32_t try_small(const WarpSmem &ws, uint32_t s, co
     ws.hs[lane] = pack_slot(hk);
     __syncwarp();
     const uint32_t hs_sa = (uint32_t)__cvta_generic_to_shared(ws.hs);
-    const uint32_t o = s <= 4   ? scan_small<4>(ws, hs_sa, s, sr, lane)
-                       : s <= 8 ? scan_small<8>(ws, hs_sa, s, sr, lane)
+    const uint32_t o = s <= 4   ? scan_blocks<4>(ws, hs_sa, s, sr, lane)
+                       : s <= 8 ? scan_blocks<8>(ws, hs_sa, s, sr, lane)
                                 : scan_quads(ws, hs_sa, s, sr, lane);
     if (o == kNone || !slots_distinct(ws.scr, hk, mine && PHB_CHECK(!mine || hk < sr.ps))) return kTryNone;
     *o_out = o;
