@@ -227,8 +227,17 @@ __global__ void __launch_bounds__(kOrderThreads, kOrderCtas) k_order(SearchArgs 
         const uint32_t p = g - d.part_base;
         const uint32_t base = a.G[(size_t)g * a.gstride], end = a.G[(size_t)(g + 1) * a.gstride];
         const uint32_t ps = end - base;
+        // The size check comes first and looks at every partition, also of a set that failed before
+        // (only a scan that timed out leaves no offsets to check): the error word then holds the
+        // lowest oversized partition, whichever CTA comes to its own first.
+        const unsigned long long e = *reinterpret_cast<volatile unsigned long long *>(&a.err[s_idx]);
         uint32_t state = 0;
-        if (fatal_before_search(*reinterpret_cast<volatile unsigned long long *>(&a.err[s_idx]))) {
+        if (e != kNoError && (uint32_t)e == PHOBIC_ERR_TIMEOUT) {
+            state = kPartSkipped;
+        } else if (ps > a.cap) {
+            report_error(&a.err[s_idx], p, PHOBIC_ERR_PARTITION_OVERFLOW);
+            state = kPartSkipped;
+        } else if (fatal_before_search(e)) {
             state = kPartSkipped;
         } else {
             if (d.part_off) {
@@ -236,10 +245,7 @@ __global__ void __launch_bounds__(kOrderThreads, kOrderCtas) k_order(SearchArgs 
                 d.part_off[p] = base - g0;
                 if (p + 1 == d.partitions) d.part_off[p + 1] = end - g0;
             }
-            if (ps > a.cap) {
-                report_error(&a.err[s_idx], p, PHOBIC_ERR_PARTITION_OVERFLOW);
-                state = kPartSkipped;
-            } else if (!PHB_CHECK(base + ps <= a.G[(size_t)a.M * a.gstride])) {
+            if (!PHB_CHECK(base + ps <= a.G[(size_t)a.M * a.gstride])) {
                 state = kPartSkipped;
             } else if (a.part_state[g] != end) {
                 // K3 placed exactly the keys K1 counted, unless the keys changed in between.
