@@ -224,8 +224,13 @@ PHOBIC_API phobic_status phobic_debug_stalled_wait(phobic_ctx *ctx, uint32_t wai
  * phobic_build_noalloc) of device-visible u64 keys with more than `index` keys runs a
  * one-thread kernel between its counting pass and its placing pass that does
  * keys[index] ^= xor_mask on the keys it builds from (the caller's device array, or the
- * context's staged copy of host keys).  The two passes then disagree and the build must
- * return PHOBIC_ERR_KEYS_CHANGED.  One shot, process-wide; xor_mask = 0 disarms it. */
+ * context's staged copy of host keys).  The two passes then disagree about the key's
+ * partition and the build must return PHOBIC_ERR_KEYS_CHANGED (a change that leaves the key in
+ * its partition gives a function of the changed keys).  A build that does K1 to K3 in one
+ * kernel (see phobic_timings) and has two partitions or more reads the keys once per
+ * partition: all its readers but the first see the changed key, and the one-thread kernel
+ * follows; it must return PHOBIC_ERR_KEYS_CHANGED whatever the key's partition, unless that
+ * is the first one before and after.  One shot, process-wide; xor_mask = 0 disarms it. */
 PHOBIC_API phobic_status phobic_debug_change_key(uint64_t index, uint64_t xor_mask);
 
 /* No counterpart in the reference.  Measurement: the integer throughput of the context's

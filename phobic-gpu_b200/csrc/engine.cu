@@ -579,7 +579,8 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
     ScanArgs sa{d_count, d_G, nullptr, (uint32_t)MS, d_tiles, reinterpret_cast<uint32_t *>(d_tiles + tiles), nsets,
                 d_err, 0, d_pcur, d_bincur, plan.stride, wshift};
     PartArgs pa{d_inter, d_bincur, d_pcur, wshift, (uint32_t)((M + (1ull << wshift) - 1) >> wshift), (uint32_t)M};
-    const bool small = nsets == 1 && !debug && !key_change && gather_fits(kind, N, M, B, cap);
+    // (The injected change needs two readers of the keys: with one partition, K1 and K3.)
+    const bool small = nsets == 1 && !debug && !(key_change && M < 2) && gather_fits(kind, N, M, B, cap);
     SearchArgs qa{d_desc, d_pb, nsets, (uint32_t)M, d_G, small ? 1u : plan.stride, d_lowers, d_bkt, d_sorted, d_dbg_sizes, B, cap,
                   k_max, d_queue, d_err, d_pcur, P};
 
@@ -594,8 +595,11 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
             PHB_TRY(record(w.ev[1]), "event");
             {
                 StageRange r("bucket_sizes, partition_offsets, key_redistribution (K1-K3)");
-                PHB_TRY(launch_gather(kind, ma, qa, d_G, d_count, d_queue + 8, s), "gather");
+                PHB_TRY(launch_gather(kind, ma, qa, d_G, d_count, d_queue + 8, s, kc_index, key_change ? kc_mask : 0),
+                        "gather");
             }
+            if (key_change)
+                PHB_TRY(launch_change_key(const_cast<void *>(hdesc[0].data), kc_index, kc_mask, s), "key change");
             for (int e = 2; e <= 4; e++) PHB_TRY(record(w.ev[e]), "event");
             {
                 StageRange r("search (K4)");

@@ -224,12 +224,13 @@ unsigned int check_line_map(bool reset);
 unsigned int check_line_part(bool reset);
 // Small builds of one set of fixed-size keys: K1, the scan and K3 in one launch (kernels_order.cu).
 // gather_fits says whether a build is one; G [M + 1] gets the partition offsets (stride 1), ends [M]
-// is scratch, *ticket starts at zero.
+// is scratch, ticket [4] (8-byte aligned) starts at zero.  change_mask (tests; u64 keys) stands for a
+// key that is written while the CTAs read: all but the first see key change_index changed by it.
 constexpr uint64_t kGatherMaxKeys = 12288;
 constexpr uint64_t kGatherMaxPartitions = 148;  // one CTA per SM
 bool gather_fits(int kind, uint64_t n, uint64_t M, uint32_t B, uint32_t cap);
 cudaError_t launch_gather(int kind, const MapArgs &m, const SearchArgs &a, uint32_t *G, uint32_t *ends, uint32_t *ticket,
-                          cudaStream_t st);
+                          cudaStream_t st, uint64_t change_index = 0, uint64_t change_mask = 0);
 unsigned int check_line_order(bool reset);
 unsigned int check_line_search(bool reset);
 // splitmix64 stream on the device: out[i] = the finalizer of seed + (i + 1) * 0x9E3779B97F4A7C15

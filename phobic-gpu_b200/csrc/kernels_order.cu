@@ -389,16 +389,27 @@ __global__ void __launch_bounds__(kOrderThreads, kOrderCtas) k_order(SearchArgs 
 // launch takes the place of K1, the scan, both partition passes and K3c; every CTA hashes every key,
 // which up to this size costs less than the launches (stage times with their events, us: 1000 keys
 // 19 against 39, 10,000 keys 37 against 45, 16,384 keys 47 against 44).
-// The CTAs read the keys at different times.  The last one to finish checks that every partition
-// ends where the next one begins; if not, the keys changed meanwhile and the build reports it (every
-// store is in bounds all the same: no CTA finds more than n keys).
+// The CTAs read the keys at different times.  The last one to finish checks that they saw the same
+// keys: every partition ends where the next one begins, and the sum over the keys that were taken
+// (key_sum) is the sum over all keys as the first CTA read them.  The sum is what tells two keys
+// that trade partitions during the build, which leave every count as it was.  If not, the build
+// reports that the keys changed (every store is in bounds all the same: no CTA finds more than n
+// keys).  A change that no CTA saw, or that every CTA saw, gives a function of the keys as read.
 __host__ __device__ __forceinline__ size_t gather_words(uint32_t B, uint32_t stage_keys) {
     return order_words(B, stage_keys) + stage_keys;
 }
 
-template <int KIND>
+// One key in the sum: all four words, so mixed that keys which differ in a pattern don't cancel.
+__device__ __forceinline__ unsigned long long key_sum(const Key4 &k) {
+    return xxh3::fold64(((uint64_t)k.lower1 << 32 | k.lower2) ^ 0x9E3779B97F4A7C15ull,
+                        ((uint64_t)k.partitioner << 32 | k.bucketer) ^ 0xD1B54A32D192ED03ull);
+}
+
+// CHANGE (tests, u64 keys): every CTA but the first reads key change_index as changed by change_mask.
+template <int KIND, bool CHANGE = false>
 __global__ void __launch_bounds__(kOrderThreads) k_gather(MapArgs m, SearchArgs a, uint32_t *G, uint32_t *ends,
-                                                         uint32_t *ticket, uint32_t stage_keys) {
+                                                         uint32_t *ticket, uint32_t stage_keys, uint32_t change_index,
+                                                         uint64_t change_mask) {
     extern __shared__ __align__(16) uint32_t smem[];
     const uint32_t B = a.buckets, tid = threadIdx.x, lane = tid & 31, n = (uint32_t)m.total_keys, p = blockIdx.x;
     uint32_t *tables = smem;
@@ -407,7 +418,9 @@ __global__ void __launch_bounds__(kOrderThreads) k_gather(MapArgs m, SearchArgs 
     uint32_t *br = reinterpret_cast<uint32_t *>(raw + stage_keys) + stage_keys / 2 + 1;  // bucket | rank << 16
     uint32_t *cnt = br + stage_keys;
     uint32_t *sched = cnt + B;
-    uint32_t *info = sched + B + 1;  // {keys taken, keys of partitions before, -, nonempty}
+    uint32_t *info = sched + B + 1;  // {keys taken, keys of partitions before, -, nonempty, sum of the keys taken}
+    unsigned long long *taken = reinterpret_cast<unsigned long long *>((reinterpret_cast<uintptr_t>(info + 4) + 7) & ~uintptr_t(7));
+    unsigned long long *sum_all = reinterpret_cast<unsigned long long *>(ticket + 2);
     const SetDesc &d = a.sets[0];
     uint32_t *pil = d.pilots + p;
     for (uint32_t i = tid; i < B; i += kOrderThreads) cnt[i] = 0;
@@ -417,13 +430,19 @@ __global__ void __launch_bounds__(kOrderThreads) k_gather(MapArgs m, SearchArgs 
 
     constexpr int U = 4;  // keys per thread and round, their loads in flight together
     uint32_t before = 0;
+    unsigned long long sum = 0;  // of the keys taken; in the first CTA less all keys, its own cancelling
     bool bad = false;
     for (uint32_t i0 = 0; i0 < n; i0 += U * kOrderThreads) {
         Key4 k[U];
 #pragma unroll
         for (int u = 0; u < U; u++) {
             const uint32_t i = i0 + u * kOrderThreads + tid;
-            k[u] = load_key<KIND>(d.data, nullptr, i < n ? i : 0);
+            if constexpr (CHANGE) {
+                const uint64_t v = __ldg(static_cast<const unsigned long long *>(d.data) + (i < n ? i : 0));
+                k[u] = key_from_hash(xxh3::hash_u64(p && i == change_index ? v ^ change_mask : v));
+            } else {
+                k[u] = load_key<KIND>(d.data, nullptr, i < n ? i : 0);
+            }
         }
 #pragma unroll
         for (int u = 0; u < U; u++) {
@@ -431,12 +450,14 @@ __global__ void __launch_bounds__(kOrderThreads) k_gather(MapArgs m, SearchArgs 
             const uint32_t gp = partition_of(k[u].partitioner, a.M);
             const bool mine = valid && gp == p;
             before += valid && gp < p;
+            if (p == 0 && valid && !mine) sum -= key_sum(k[u]);
             const uint32_t ball = __ballot_sync(kFullMask, mine);
             if (!ball) continue;
             uint32_t at = 0;
             if (lane == (uint32_t)__ffs(ball) - 1) at = atomicAdd(&info[0], (uint32_t)__popc(ball));
             at = __shfl_sync(kFullMask, at, __ffs(ball) - 1) + __popc(ball & lanemask_lt());
             if (!mine) continue;
+            if (p) sum += key_sum(k[u]);
             const uint32_t b = bucket_of(k[u].bucketer, m.fulcs);
             bad |= b >= B;
             if (at < stage_keys) {  // more only where the partition exceeds the search's capacity
@@ -447,7 +468,11 @@ __global__ void __launch_bounds__(kOrderThreads) k_gather(MapArgs m, SearchArgs 
         }
     }
     before = __reduce_add_sync(kFullMask, before);
-    if (lane == 0 && before) atomicAdd(&info[1], before);
+    for (int x = 16; x; x >>= 1) sum += __shfl_xor_sync(kFullMask, sum, x);
+    if (lane == 0) {
+        if (before) atomicAdd(&info[1], before);
+        atomicAdd(taken, sum);
+    }
     if (bad) report_error(&a.err[0], 0, PHOBIC_ERR_INVALID);
     __syncthreads();
 
@@ -503,11 +528,12 @@ __global__ void __launch_bounds__(kOrderThreads) k_gather(MapArgs m, SearchArgs 
     }
     if (tid == 0) {
         a.part_state[p] = state;
+        atomicAdd(sum_all, *taken);
         __threadfence();
         if (atomicAdd(ticket, 1u) == a.M - 1) {
             __threadfence();
             const volatile uint32_t *g = G, *e = ends;
-            bool same = g[0] == 0;
+            bool same = g[0] == 0 && *reinterpret_cast<volatile unsigned long long *>(sum_all) == 0;
             for (uint32_t q = 0; q < a.M; q++) same &= e[q] == (q + 1 < a.M ? g[q + 1] : n);
             if (!same)
                 for (uint32_t q = 0; q < a.M; q++) a.part_state[q] = kPartSkipped | PHOBIC_ERR_KEYS_CHANGED;
@@ -527,19 +553,21 @@ bool gather_fits(int kind, uint64_t n, uint64_t M, uint32_t B, uint32_t cap) {
     return kind != PHOBIC_KEYS_STRINGS && gather_smem(n, M, B, cap, &stage) != 0;
 }
 
-template <int KIND>
+template <int KIND, bool CHANGE = false>
 static cudaError_t launch_gather_kind(const MapArgs &m, const SearchArgs &a, uint32_t *G, uint32_t *ends,
-                                      uint32_t *ticket, cudaStream_t st) {
+                                      uint32_t *ticket, cudaStream_t st, uint32_t index = 0, uint64_t mask = 0) {
     uint32_t stage = 0;
     const size_t smem = gather_smem(m.total_keys, a.M, a.buckets, a.cap, &stage);
-    const cudaError_t e = allow_dynamic_smem(k_gather<KIND>, smem);
+    const cudaError_t e = allow_dynamic_smem(k_gather<KIND, CHANGE>, smem);
     if (e != cudaSuccess) return e;
-    k_gather<KIND><<<a.M, kOrderThreads, smem, st>>>(m, a, G, ends, ticket, stage);
+    k_gather<KIND, CHANGE><<<a.M, kOrderThreads, smem, st>>>(m, a, G, ends, ticket, stage, index, mask);
     return cudaGetLastError();
 }
 
 cudaError_t launch_gather(int kind, const MapArgs &m, const SearchArgs &a, uint32_t *G, uint32_t *ends, uint32_t *ticket,
-                          cudaStream_t st) {
+                          cudaStream_t st, uint64_t change_index, uint64_t change_mask) {
+    if (change_mask)  // u64 keys (take_key_change)
+        return launch_gather_kind<PHOBIC_KEYS_U64, true>(m, a, G, ends, ticket, st, (uint32_t)change_index, change_mask);
     switch (kind) {
     case PHOBIC_KEYS_U64: return launch_gather_kind<PHOBIC_KEYS_U64>(m, a, G, ends, ticket, st);
     case PHOBIC_KEYS_BYTES16: return launch_gather_kind<PHOBIC_KEYS_BYTES16>(m, a, G, ends, ticket, st);

@@ -40,3 +40,36 @@ def test_the_lowest_of_adjacent_oversized_partitions_is_reported(phobic):
         for _ in range(10):
             _, st = phobic.build_batch(ctx, [good, k4], cfg, kind=phobic.KEYS_PREHASHED)
             assert st == [phobic.OK, phobic.ERR_PARTITION_OVERFLOW] and f"set 1, partition {first})" in ctx.last_error
+
+
+@pytest.mark.parametrize("way", ["down", "up", "from_first", "to_first", "same"])
+def test_keys_changed_during_a_small_build_are_reported(phobic, way):
+    """A small build reads its keys once per partition; here all readers but the first see one key
+    changed (phobic_debug_change_key): moved to another partition, or, what no count can tell, to
+    another place of its own partition.  The build of the keys as they then are is the oracle's."""
+    torch = pytest.importorskip("torch")
+    n = 9_000
+    cfg = phobic.MPHFconfig(5.0, 2048)
+    M = cfg.partitions(n)
+    keys = keygen.splitmix64(73, n)
+
+    def part(k):
+        return (O.hash_keys(k, "u64")[:, 0].astype(np.uint64) * M >> np.uint64(32)).astype(int)
+
+    old = part(keys)
+    new = part(keys ^ np.uint64(0xFFFF))
+    pick = {"down": (old > new) & (new > 0), "up": (old < new) & (old > 0), "from_first": (old == 0) & (new > 0),
+            "to_first": (new == 0) & (old > 0), "same": (old == new) & (old > 0)}[way]
+    index = int(np.flatnonzero(pick)[-1])
+    dk = torch.from_numpy(keys.view(np.int64).copy()).cuda()
+    with phobic.Context(0) as ctx:
+        phobic.debug_change_key(index, 0xFFFF)
+        with pytest.raises(phobic.PhobicError) as e:
+            ctx.build(dk, cfg)
+        assert e.value.status == phobic.ERR_KEYS_CHANGED
+        now = dk.cpu().numpy().view(np.uint64)
+        assert np.flatnonzero(now != keys).tolist() == [index] and now[index] == keys[index] ^ np.uint64(0xFFFF)
+        got = ctx.build(now, cfg)
+        want = O.build(O.hash_keys(now, "u64"), 2048, cfg.bucketCountPerPartition, cfg.getFulcs())
+        assert got.timings["kernels"] == 2
+        assert (got.pilots == want["pilots"]).all() and (got.partition_offsets == want["offsets"]).all()
