@@ -189,6 +189,8 @@ phobic_status run_encode_gpu(Worker &w, DeviceArena &out_arena, int pilot_encode
     const bool mono = pilot_encoder == 3;
     const uint32_t cols = mono ? 1u : (uint32_t)B;
     PHB_TRY(cudaSetDevice(w.device), "cudaSetDevice");
+    phobic_status st = settle(w, err);
+    if (st != PHOBIC_OK) return st;
     PHB_TRY(w.pinned.reserve(4096), "pinned");
     cudaStream_t s = w.stream;
 
@@ -237,14 +239,15 @@ phobic_status run_encode_gpu(Worker &w, DeviceArena &out_arena, int pilot_encode
     unsigned long long *h_info = static_cast<unsigned long long *>(w.pinned.data());
     PHB_TRY(cudaMemcpyAsync(h_info, d_info, 16, cudaMemcpyDeviceToHost, s), "D2H size");
     PHB_TRY(cudaEventRecord(w.ev[7], s), "event");
-    phobic_status st = wait_event(w.ev[7], w.timeout_ms, err);
-    if (st != PHOBIC_OK) return st;
+    if ((st = wait_event(w.ev[7], w.timeout_ms, err)) != PHOBIC_OK) return st;
+    w.unsettled = false;
     const uint64_t total = h_info[0], n = h_info[1];
     *size = total;
     // getBitsPerKey (mphf.hpp:88-91): encoder bits (8 per serialised byte), fulcrums and partition count.
     if (bits_per_key) *bits_per_key = n ? (double)(float(total * 8 + 32 * (uint64_t)kFulcrums + 32 * P) / float(n)) : 0.0;
     if (!out || (direct && total <= cap)) return PHOBIC_OK;
 
+    w.unsettled = true;
     PHB_TRY(out_arena.reserve(total), "device output");
     out_arena.reset();
     uint8_t *d_out = static_cast<uint8_t *>(out_arena.take(total));
@@ -254,7 +257,8 @@ phobic_status run_encode_gpu(Worker &w, DeviceArena &out_arena, int pilot_encode
         PHB_TRY(cudaMemcpyAsync(out, d_out, ncopy, out_on_device ? cudaMemcpyDeviceToDevice : cudaMemcpyDeviceToHost, s),
                 "copy out");
     PHB_TRY(cudaEventRecord(w.ev[7], s), "event");
-    return wait_event(w.ev[7], w.timeout_ms, err);
+    if ((st = wait_event(w.ev[7], w.timeout_ms, err)) == PHOBIC_OK) w.unsettled = false;
+    return st;
 }
 
 }  // namespace phobicb200

@@ -250,6 +250,15 @@ phobic_status wait_stream(cudaStream_t s, uint64_t timeout_ms, std::string *err)
     return bounded_wait([s] { return cudaStreamQuery(s); }, timeout_ms, err);
 }
 
+phobic_status settle(Worker &w, std::string *err) {
+    if (w.unsettled) {
+        const phobic_status st = wait_stream(w.stream, w.timeout_ms, err);
+        if (st != PHOBIC_OK) return st;
+    }
+    w.unsettled = true;
+    return PHOBIC_OK;
+}
+
 uint64_t env_timeout_ms() {
     if (const char *t = std::getenv("PHOBIC_TIMEOUT_MS")) {
         char *end = nullptr;
@@ -460,6 +469,7 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
     const size_t tab_desc = align256(sizeof(SetDesc) * nsets), tab_kb = align256(8 * (nsets + 1)),
                  tab_pb = align256(8 * (nsets + 1)), tab_fulcs = align256(4 * kFulcrums), tab_err = align256(8 * nsets);
     const size_t tab_in = tab_desc + tab_kb + tab_pb + tab_fulcs;
+    if ((st = settle(w, err)) != PHOBIC_OK) return st;
     PHB_TRY(w.pinned.reserve(tab_in + tab_err), "pinned table");
     char *tab = static_cast<char *>(w.pinned.data());
     SetDesc *hdesc = reinterpret_cast<SetDesc *>(tab);
@@ -743,6 +753,7 @@ phobic_status finish_sets(Worker &w, phobic_status *statuses, phobic_timings *t,
         st = wait_event(w.ev[6], w.timeout_ms, err);
     }
     if (st != PHOBIC_OK) return st;
+    w.unsettled = false;
     if (!w.pending_copies.empty()) {
         StageRange r("copy results to pageable memory");
         copy_out(w.pending_copies, static_cast<const char *>(w.stage.data()));
@@ -778,6 +789,8 @@ phobic_status finish_sets(Worker &w, phobic_status *statuses, phobic_timings *t,
 
 phobic_status run_stalled_wait(Worker &w, uint32_t wait_ms, phobic_status *observed, std::string *err) {
     PHB_TRY(cudaSetDevice(w.device), "cudaSetDevice");
+    phobic_status st = settle(w, err);
+    if (st != PHOBIC_OK) return st;
     const uint32_t m = 2 * kScanTile;  // two tiles: tile 1 waits on tile 0, which never runs
     w.arena.reset();
     PHB_TRY(w.arena.reserve(align256(4 * m) + align256(4 * (m + 1)) + align256(8 * 2 + 8) + align256(8) + 4096),
@@ -794,12 +807,12 @@ phobic_status run_stalled_wait(Worker &w, uint32_t wait_ms, phobic_status *obser
     ScanArgs sa{d_in, d_out, nullptr, m, d_tiles, reinterpret_cast<uint32_t *>(d_tiles + 2), 1, d_err,
                 (unsigned long long)wait_ms * 1000000ull};
     PHB_TRY(launch_scan_stalled(sa, 1, s), "stalled scan");
-    PHB_TRY(w.pinned.reserve(4096), "pinned");
+    PHB_TRY(w.pinned.reserve(4096), "pinned");  // settled above
     unsigned long long *h = static_cast<unsigned long long *>(w.pinned.data());
     PHB_TRY(cudaMemcpyAsync(h, d_err, 8, cudaMemcpyDeviceToHost, s), "D2H");
     PHB_TRY(cudaEventRecord(w.ev[7], s), "event");
-    phobic_status st = wait_event(w.ev[7], w.timeout_ms, err);
-    if (st != PHOBIC_OK) return st;
+    if ((st = wait_event(w.ev[7], w.timeout_ms, err)) != PHOBIC_OK) return st;
+    w.unsettled = false;
     *observed = *h == kNoError ? PHOBIC_OK : (phobic_status)(uint32_t)*h;
     return PHOBIC_OK;
 }
@@ -817,6 +830,7 @@ phobic_status run_query(Worker &w, const phobic_keys *keys, const phobic_params 
     const uint64_t n = keys->n;
     const uint32_t B = params->buckets;
     PHB_TRY(cudaSetDevice(w.device), "cudaSetDevice");
+    if ((st = settle(w, err)) != PHOBIC_OK) return st;
     PHB_TRY(w.pinned.reserve(256 + 4 * kFulcrums), "pinned");
     unsigned long long *hword = static_cast<unsigned long long *>(w.pinned.data());
     uint64_t bytes = 8192 + align256(4 * kFulcrums) + align256(8) + align256(4 * (size_t)B * partitions) +
@@ -843,7 +857,7 @@ phobic_status run_query(Worker &w, const phobic_keys *keys, const phobic_params 
         }
     }
     uint32_t *d_fulcs = static_cast<uint32_t *>(w.arena.take(4 * kFulcrums));
-    char *fulcs = static_cast<char *>(w.pinned.data()) + 256;  // free: every call waits for its work
+    char *fulcs = static_cast<char *>(w.pinned.data()) + 256;  // free: the worker is settled
     std::memcpy(fulcs, params->fulcrums, 4 * kFulcrums);
     PHB_TRY(cudaMemcpyAsync(d_fulcs, fulcs, 4 * kFulcrums, cudaMemcpyHostToDevice, s), "H2D fulcrums");
     unsigned long long *d_bad = static_cast<unsigned long long *>(w.arena.take(8));
@@ -881,6 +895,7 @@ phobic_status run_query(Worker &w, const phobic_keys *keys, const phobic_params 
     }
     PHB_TRY(cudaEventRecord(w.ev[7], s), "event");
     if ((st = wait_event(w.ev[7], w.timeout_ms, err)) != PHOBIC_OK) return st;
+    w.unsettled = false;
     if (bad) *bad = *hword + (n > n_built ? n - n_built : n_built - n);
     return PHOBIC_OK;
 }

@@ -85,6 +85,9 @@ struct Worker {
     std::vector<uint64_t> graph_key;      // launch identity of the last build
     cudaGraphExec_t graph_exec = nullptr;  // captured stages of graph_key, if any
     bool pending_graph = false;           // the last enqueued build replayed graph_exec
+    // Work of an earlier call may still be queued: its wait ran out, or it failed midway.  That work
+    // reads and writes the pinned buffers, so settle() waits for it before they are used again.
+    bool unsettled = false;
     void drop_graph();
 
     phobic_status init(int device, std::string *err);
@@ -117,6 +120,9 @@ phobic_status finish_sets(Worker &w, phobic_status *statuses, phobic_timings *t,
 phobic_status wait_event(cudaEvent_t ev, uint64_t timeout_ms, std::string *err);
 // The same bounded wait on all work queued on a stream (cudaStreamQuery).
 phobic_status wait_stream(cudaStream_t s, uint64_t timeout_ms, std::string *err);
+// Before a call uses the worker's pinned buffers: waits (bounded) for what an earlier call left queued.
+// The worker is unsettled from then on until the call has waited for its own work.
+phobic_status settle(Worker &w, std::string *err);
 // Bound of the host-side waits: PHOBIC_TIMEOUT_MS from the environment, else 120 s.
 uint64_t env_timeout_ms();
 

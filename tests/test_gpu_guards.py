@@ -73,3 +73,73 @@ def test_keys_changed_during_a_small_build_are_reported(phobic, way):
         want = O.build(O.hash_keys(now, "u64"), 2048, cfg.bucketCountPerPartition, cfg.getFulcs())
         assert got.timings["kernels"] == 2
         assert (got.pilots == want["pilots"]).all() and (got.partition_offsets == want["offsets"]).all()
+
+
+def test_calls_after_a_timeout_leave_the_queued_build_alone(phobic, monkeypatch):
+    """A build that timed out stays queued and still reads its pinned tables.  Calls that follow
+    (a query with another configuration, a build of other keys) wait for it, time out like it
+    while it is held back, and neither disturb it nor take over its status.  The work is held
+    back by a bounded sleep kernel on the context's stream (about 0.3 s)."""
+    torch = pytest.importorskip("torch")
+    cfg, other = phobic.MPHFconfig(7.0, 2500), phobic.MPHFconfig(4.0, 1000)
+    keys, twice = keygen.splitmix64(81, 100_000), keygen.splitmix64(82, 100_000)
+    twice[9] = twice[8]
+
+    def oracle(k, c):
+        return O.build(O.hash_keys(k, "u64"), c.partitionSize, c.bucketCountPerPartition, c.getFulcs())
+
+    want, want_other = oracle(keys, cfg), oracle(keys, other)
+    dk, dt = (torch.from_numpy(k.view(np.int64)).cuda() for k in (keys, twice))
+
+    def arrays(c):
+        m = c.partitions(len(keys))
+        return (torch.zeros(m * c.bucketCountPerPartition, dtype=torch.int32, device="cuda"),
+                torch.zeros(m + 1, dtype=torch.int32, device="cuda"))
+
+    def same(out, w):
+        return ((out[0].cpu().numpy().view(np.uint32) == w["pilots"]).all()
+                and (out[1].cpu().numpy().view(np.uint32) == w["offsets"]).all())
+
+    first, late, built = arrays(cfg), arrays(cfg), arrays(other)
+    with phobic.Context(0) as warm:  # loads every kernel
+        r_other = warm.build(dk, other, out=built)
+        slots = warm.query(dk, other, r_other)
+        warm.build(dk, cfg, out=late)
+        phobic.encode_gpu(warm, r_other, other, "interleaved_compact", "diff")
+    assert same(built, want_other)
+    monkeypatch.setenv("PHOBIC_TIMEOUT_MS", "40")
+    with phobic.Context(0) as ctx:
+        monkeypatch.delenv("PHOBIC_TIMEOUT_MS")
+        for _ in range(2):  # arenas at their sizes
+            ctx.build(dk, cfg, out=late)
+            assert torch.equal(ctx.query(dk, other, r_other), slots)
+        for t in late:
+            t.zero_()
+        torch.cuda.synchronize()
+
+        def timed_out(call):
+            with pytest.raises(phobic.PhobicError) as e:
+                call()
+            assert e.value.status == phobic.ERR_TIMEOUT
+
+        with torch.cuda.stream(torch.cuda.ExternalStream(ctx.stream_handle())):
+            torch.cuda._sleep(600_000_000)
+        timed_out(lambda: ctx.build(dk, cfg, out=first))
+        timed_out(lambda: ctx.query(dk, other, r_other))
+        timed_out(lambda: ctx.build(dt, cfg, out=late))
+        timed_out(lambda: phobic.encode_gpu(ctx, r_other, other, "interleaved_compact", "diff"))
+        torch.cuda.synchronize()
+        assert same(first, want)
+        assert not late[0].any()  # never queued
+        assert torch.equal(ctx.query(dk, other, r_other), slots)
+        # A failing build left queued does not lend its status to the next one.
+        with torch.cuda.stream(torch.cuda.ExternalStream(ctx.stream_handle())):
+            torch.cuda._sleep(200_000_000)
+        timed_out(lambda: ctx.build(dt, cfg, out=first))
+        for _ in range(20):
+            try:
+                ctx.build(dk, cfg, out=late)
+                break
+            except phobic.PhobicError as e:
+                assert e.status == phobic.ERR_TIMEOUT
+        assert same(late, want)
