@@ -659,7 +659,7 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
         w.drop_graph();  // also when the caller is capturing the stream: the stages join that capture
     } else {
         // Everything the launches depend on: sizes, parameters, plan, shape and every buffer.
-        std::vector<uint64_t> key{nsets, (uint64_t)kind, N, M, B, cap, k_max, plan.stride, plan.chunk, plan.grid,
+        std::vector<uint64_t> key{nsets, (uint64_t)kind, N, M, P, B, cap, k_max, plan.stride, plan.chunk, plan.grid,
                                   (uint64_t)plan.chunked | (uint64_t)plan.narrow << 1, wshift, tiles,
                                   (uint64_t)shape.group, (uint64_t)shape.pipeline, (uint64_t)w.sm_count, (uint64_t)small};
         for (const void *p : {(const void *)d_fulcs, (const void *)d_desc, (const void *)d_kb, (const void *)d_pb,

@@ -114,6 +114,22 @@ def test_changed_launches_are_never_replayed(phobic):
                 assert e.value.status == want["status"]
 
 
+def test_another_partition_size_is_captured_anew(phobic):
+    """Partition sizes that give the same partitions, buckets and capacity still give other launches:
+    the bucket order's stage and the search's shape go by the partition size."""
+    one, two = phobic.MPHFconfig(5.0, 1900), phobic.MPHFconfig(5.0, 1897)
+    two.params.max_partition_size = one.params.max_partition_size
+    assert one.bucketCountPerPartition == two.bucketCountPerPartition
+    keys = keygen.splitmix64(14, 20_000)
+    with phobic.Context(0) as ctx:
+        replays = []
+        for cfg in (one, one, two, two, one):
+            got = ctx.build(keys, cfg)
+            assert got.partitions == 11 and (got.pilots == oracle(keys, cfg)["pilots"]).all()
+            replays.append(got.timings["graph_replays"])
+    assert replays == [0, 1, 0, 1, 0]
+
+
 def test_batch_builds_replay_and_match(phobic):
     cfg = phobic.MPHFconfig(6.0, 2048)
     sets = [keygen.splitmix64(50 + i, 3000 * (i + 1)) for i in range(6)]
