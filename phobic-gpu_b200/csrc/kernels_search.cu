@@ -911,7 +911,8 @@ __device__ __forceinline__ void pipeline(const WarpSmem &ws, const uint2 *so, co
         read(j + 3 * W);
         Seek<NR> f;
         f.kb = f.k = f.o = f.h = 0;
-        uint32_t st = *status, q = 0, at = 0, bit = 0;
+        // One lane reads the status, which another warp may be writing: the warp agrees on what it saw.
+        uint32_t st = __shfl_sync(kFullMask, lane == 0 ? *status : 0u, 0), q = 0, at = 0, bit = 0;
         bool turn = false, seek = st == PHOBIC_OK, on = false;
 #pragma unroll 1
         for (;;) {
