@@ -275,7 +275,7 @@ phobic_status phobic_debug_checks(phobic_ctx *ctx, int *compiled, uint32_t *line
 #endif
     lines[0] = check_line_map(reset != 0);
     const unsigned int part = check_line_part(reset != 0), order = check_line_order(reset != 0);
-    lines[1] = part ? part : order;
+    lines[1] = part ? part : order ? kOrderCheckBase + order : 0u;
     lines[2] = check_line_search(reset != 0);
     return PHOBIC_OK;
 }

@@ -232,6 +232,9 @@ bool gather_fits(int kind, uint64_t n, uint64_t M, uint32_t B, uint32_t cap);
 cudaError_t launch_gather(int kind, const MapArgs &m, const SearchArgs &a, uint32_t *G, uint32_t *ends, uint32_t *ticket,
                           cudaStream_t st, uint64_t change_index = 0, uint64_t change_mask = 0);
 unsigned int check_line_order(bool reset);
+// phobic_debug_checks has one word for the partition and the order kernels: a line of the latter
+// comes back with this added (no file is that long).
+constexpr unsigned int kOrderCheckBase = 100000;
 unsigned int check_line_search(bool reset);
 // splitmix64 stream on the device: out[i] = the finalizer of seed + (i + 1) * 0x9E3779B97F4A7C15
 // (synthetic keys of the autotuner).

@@ -378,7 +378,8 @@ class Context:
 
     def checks(self, reset: bool = False) -> tuple[bool, list[int]]:
         """(checked library?, source lines of the first failed bounds check in the
-        key-mapping, partition and search kernels; 0 = none)."""
+        key-mapping, partition and search kernels; 0 = none).  The second word is also the
+        bucket-order kernels': 100,000 + the line in their file."""
         compiled = C.c_int32()
         lines = (U32 * 3)()
         check(_lib().phobic_debug_checks(self.handle, C.byref(compiled), lines, int(reset)), self)
