@@ -188,6 +188,8 @@ __device__ __forceinline__ Key4 load_key(const void *data, const uint64_t *offse
 
 // Shared-memory bytes one warp of K4 needs for a partition capacity and bucket count.
 size_t search_warp_smem(uint32_t buckets, uint32_t cap);
+// Shared-memory bytes K3c needs for a bucket count (without a stage of keys).
+size_t order_smem(uint32_t buckets);
 // Whether the build takes these parameters (they bound the shared memory of K3c and K4).
 bool search_accepts(uint32_t buckets, uint32_t cap);
 // K3c: size check, bucket sizes, search order and bucket-ordered keys of every partition.

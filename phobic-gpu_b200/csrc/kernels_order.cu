@@ -575,6 +575,8 @@ cudaError_t launch_gather(int kind, const MapArgs &m, const SearchArgs &a, uint3
     }
 }
 
+size_t order_smem(uint32_t buckets) { return 4 * order_words(buckets, 0); }
+
 unsigned int check_line_order(bool reset) { return read_check_line(reset); }
 
 cudaError_t launch_order(const SearchArgs &a, int sm_count, cudaStream_t st) {

@@ -1066,15 +1066,19 @@ unsigned int check_line_search(bool reset) { return read_check_line(reset); }
 
 size_t search_warp_smem(uint32_t buckets, uint32_t cap) { return 4 * warp_words(buckets, cap); }
 
-// The bound is the shared memory of a warp that also sorted its partition (packed u16 tables of
-// bucket sizes and cursors, two of 256 size bins, slots, collision scratch, schedule and
-// bitmap); K3c and K4, which share that work, both need less.
+// The rule for what is accepted is the shared memory of a warp that also sorts its partition (packed
+// u16 tables of bucket sizes and cursors, two of 256 size bins, slots, collision scratch, schedule
+// and bitmap).  K3c without its stage and K4 take more than that where it is far below the limit
+// (the bitmap of pairs: 46 KB at 65,535 slots and 1,000 buckets against 32) and less near it (two words a
+// bucket each against two and a half), so the last two conditions refuse nothing that the first one
+// accepts; they hold the layouts to it.
 bool search_accepts(uint32_t buckets, uint32_t cap) {
     if (cap > 65535 || buckets > 65535) return false;
     const size_t half = (buckets + 1) / 2, reach = (cap - 1) / 32 + 32 * ((cap + 1023) / 1024) + 2,
                  occ = (2 * cap + 31) / 32 + 2;
     const size_t words = std::max(half + 256, (size_t)kHsWords + scr_words(cap)) + half + buckets + std::max(reach, occ);
-    return 4 * ((words + 3) & ~size_t(3)) <= kSearchSmemLimit;
+    return 4 * ((words + 3) & ~size_t(3)) <= kSearchSmemLimit && search_warp_smem(buckets, cap) <= kSearchSmemLimit &&
+           order_smem(buckets) <= kSearchSmemLimit;
 }
 
 int search_warps_per_cta(uint32_t buckets, uint32_t cap) {

@@ -134,3 +134,27 @@ def test_shipped_tuning_table_is_well_formed(phobic):
         groups.setdefault((dev, P, B, cap), []).append(cls)
     for key, classes in groups.items():
         assert classes == sorted(classes) and len(set(classes)) == len(classes), key
+
+
+@pytest.mark.parametrize("cap", [1, 33, 1024, 3072, 16_384, 50_001, 65_535])
+def test_accepted_bucket_counts_follow_the_documented_rule(phobic, cap):
+    """Buckets and capacity are accepted by the shared memory of a warp that also sorts its partition,
+    whatever the kernels' present layouts take: on both sides of the largest bucket count.  (A call
+    beyond the static array's keys ends with PHOBIC_ERR_BUDGET once its parameters are accepted.)"""
+    def words(B):
+        half, scr = (B + 1) // 2, (cap + 31) // 32 + 1
+        bitmap = max((cap - 1) // 32 + 32 * ((cap + 1023) // 1024) + 2, (2 * cap + 31) // 32 + 2)
+        return (max(half + 256, 260 + scr) + half + B + bitmap + 3) & ~3
+
+    def accepted(B):
+        p = phobic.MPHFconfig(5.0, 2048).params
+        p.buckets, p.max_partition_size, p.fulcrums[2047] = B, cap, (B << 16) & 0xFFFFFFFF
+        keys = phobic.Keys(phobic.KEYS_U64, 1, 1 << 31, 4096, None)
+        r = phobic.Result(1, 4096, 4096)
+        st = phobic.lib().phobic_build_noalloc(C.byref(keys), C.byref(p), C.byref(r), None)
+        assert st in (phobic.ERR_INVALID, phobic.ERR_BUDGET)
+        return st == phobic.ERR_BUDGET
+
+    top = max(B for B in range(1, 65_536) if 4 * words(B) <= 227 * 1024)
+    for B in (1, 512, 513, top - 1, top, top + 1, 65_535):
+        assert accepted(B) == (4 * words(B) <= 227 * 1024), B
