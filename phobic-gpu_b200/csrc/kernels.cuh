@@ -71,7 +71,7 @@ struct MapPlan {
     uint32_t stride;  // count-matrix entries per partition (chunks, or 1)
     uint32_t grid;
     uint64_t chunk;   // keys per CTA (chunked plan)
-    bool narrow;      // chunked with 16-bit counters: K1 counting only, launch_scatter refuses it
+    bool narrow;      // chunked with 16-bit counters
 };
 MapPlan plan_map(uint64_t total_keys, uint64_t partitions, int sm_count);
 

@@ -10,13 +10,14 @@
 // The bucket order inside a partition is produced later, in shared memory, by K3c.
 //
 // Two plans (plan_map):
-//   chunked  CTA c counts (K1) and places (K3) the keys of one contiguous chunk
-//            with a shared-memory counter per partition; the only global traffic
-//            is the streamed keys, one column of the count matrix and the record
-//            stores.  Used while all partitions' counters fit in shared memory,
-//            32-bit up to 52K partitions, packed 16-bit (counting) up to 104K.
+//   chunked  K1: CTA c counts the keys of one contiguous chunk with a shared-memory
+//            counter per partition; the only global traffic is the streamed keys and
+//            one column of the count matrix.  Used while all partitions' counters fit
+//            in shared memory, 32-bit up to 52K partitions, packed 16-bit up to 104K.
 //   global   one counter per partition in global memory, a reduction per key in
-//            K1 and an atomic add per key in K3 (builds with more partitions).
+//            K1 (builds with more partitions) and an atomic add per key in K3.
+// K3 in one pass by cursors per partition is the no-allocation build's; the others partition
+// in two passes (kernels_part.cu).
 #include "kernels.cuh"
 
 namespace phobicb200 {
@@ -136,23 +137,18 @@ static __device__ __forceinline__ void credit_wrap(const MapArgs &a, uint32_t c,
         atomicAdd(&a.counts[(size_t)(g + 1) * a.stride + c], (old >> 16) == 0xFFFFu ? 65535u : 0xFFFFFFFFu);
 }
 
-// Chunked plan: CTA c owns keys [c * chunk, (c + 1) * chunk).  K1 counts them per
-// partition in shared memory and writes column c of the count matrix; K3 loads
-// column c of its exclusive scan as cursors and hands out slots with
-// shared-memory atomics.  NARROW (K1 only) packs two 16-bit counters per word.
-template <int KIND, bool SCATTER, bool NARROW>
+// Chunked plan: CTA c owns keys [c * chunk, (c + 1) * chunk), counts them per partition in
+// shared memory and writes column c of the count matrix.  NARROW packs two 16-bit counters per word.
+template <int KIND, bool NARROW>
 __global__ void __launch_bounds__(kChunkThreads, 1) k_chunk(MapArgs a) {
-    static_assert(!(SCATTER && NARROW), "slots need 32-bit cursors");
     extern __shared__ __align__(16) uint32_t smem[];
     __shared__ uint32_t wrapped;       // a 16-bit counter wrapped in this CTA
     uint32_t *sf = smem;               // [kFulcrums]
     uint32_t *cnt = smem + kFulcrums;  // [M], or [(M + 1) / 2] packed
-    constexpr bool kReadMapped = SCATTER && KIND == PHOBIC_KEYS_STRINGS;
     const uint32_t c = blockIdx.x;
-    if (!kReadMapped)
-        for (uint32_t i = threadIdx.x; i < kFulcrums; i += blockDim.x) sf[i] = a.fulcs[i];
+    for (uint32_t i = threadIdx.x; i < kFulcrums; i += blockDim.x) sf[i] = a.fulcs[i];
     const uint32_t words = NARROW ? (a.M + 1) / 2 : a.M;
-    for (uint32_t g = threadIdx.x; g < words; g += blockDim.x) cnt[g] = SCATTER ? a.counts[(size_t)g * a.stride + c] : 0u;
+    for (uint32_t g = threadIdx.x; g < words; g += blockDim.x) cnt[g] = 0u;
     if (threadIdx.x == 0) wrapped = 0u;
     __syncthreads();
 
@@ -162,7 +158,7 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_chunk(MapArgs a) {
     uint32_t bad_set = 0xFFFFFFFFu;
     // u64 keys of one set (the plain build): all of an iteration's key loads are
     // issued before any of them is hashed, so kUnroll loads per thread are in flight.
-    constexpr bool kRawU64 = KIND == PHOBIC_KEYS_U64 && !kReadMapped;
+    constexpr bool kRawU64 = KIND == PHOBIC_KEYS_U64;
     const bool raw_u64 = kRawU64 && a.nsets == 1;
     const unsigned long long *keys64 = kRawU64 ? static_cast<const unsigned long long *>(a.sets[0].data) : nullptr;
     const uint32_t parts0 = a.sets[0].partitions;
@@ -184,10 +180,8 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_chunk(MapArgs a) {
                 gp[u] = partition_of(k.partitioner, parts0);
                 b[u] = bucket_of(k.bucketer, sf);
                 l1[u] = k.lower1, l2[u] = k.lower2;
-                if (!SCATTER) {
-                    if (b[u] >= a.buckets && bad_set == 0xFFFFFFFFu) bad_set = 0;
-                    if (a.debug_keys) a.debug_keys[g] = make_uint4(k.partitioner, k.bucketer, k.lower1, k.lower2);
-                }
+                if (b[u] >= a.buckets && bad_set == 0xFFFFFFFFu) bad_set = 0;
+                if (a.debug_keys) a.debug_keys[g] = make_uint4(k.partitioner, k.bucketer, k.lower1, k.lower2);
             }
         } else {
 #pragma unroll
@@ -195,28 +189,15 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_chunk(MapArgs a) {
             const uint64_t g = g0 + (uint64_t)u * kChunkThreads;
             gp[u] = 0xFFFFFFFFu;
             if (g >= hi) continue;
-            map_key<KIND, kReadMapped>(a, sc, sf, g, gp[u], b[u], l1[u], l2[u]);
-            if (!SCATTER) {
-                if (b[u] >= a.buckets && bad_set == 0xFFFFFFFFu) bad_set = sc.s;
-                if (a.debug_keys) {
-                    Key4 k = load_key<KIND>(sc.data, sc.offsets, g - sc.lo);
-                    a.debug_keys[g] = make_uint4(k.partitioner, k.bucketer, k.lower1, k.lower2);
-                }
+            map_key<KIND, false>(a, sc, sf, g, gp[u], b[u], l1[u], l2[u]);
+            if (b[u] >= a.buckets && bad_set == 0xFFFFFFFFu) bad_set = sc.s;
+            if (a.debug_keys) {
+                Key4 k = load_key<KIND>(sc.data, sc.offsets, g - sc.lo);
+                a.debug_keys[g] = make_uint4(k.partitioner, k.bucketer, k.lower1, k.lower2);
             }
         }
         }
-        if constexpr (SCATTER) {
-            uint32_t slot[kUnroll];
-#pragma unroll
-            for (int u = 0; u < kUnroll; u++)
-                if (gp[u] != 0xFFFFFFFFu) slot[u] = PHB_CHECK(gp[u] < a.M) ? atomicAdd(&cnt[gp[u]], 1u) : 0u;
-#pragma unroll
-            for (int u = 0; u < kUnroll; u++) {
-                if (gp[u] == 0xFFFFFFFFu) continue;
-                a.lowers[slot[u]] = make_uint2(l1[u], l2[u]);
-                a.bkt[slot[u]] = (uint16_t)b[u];
-            }
-        } else if constexpr (NARROW) {
+        if constexpr (NARROW) {
             uint32_t old[kUnroll];
 #pragma unroll
             for (int u = 0; u < kUnroll; u++) {
@@ -241,21 +222,19 @@ __global__ void __launch_bounds__(kChunkThreads, 1) k_chunk(MapArgs a) {
         }
     }
     if (bad_set != 0xFFFFFFFFu) report_error(&a.err[bad_set], 0, PHOBIC_ERR_INVALID);
-    if (!SCATTER) {
-        __syncthreads();
-        if (NARROW) {
-            // After a wrap the column already holds the credited 65536s: add to it.
-            const bool add = wrapped != 0u;
-            for (uint32_t g = threadIdx.x; g < a.M; g += blockDim.x) {
-                const uint32_t v = (cnt[g >> 1] >> ((g & 1u) << 4)) & 0xFFFFu;
-                if (add)
-                    atomicAdd(&a.counts[(size_t)g * a.stride + c], v);
-                else
-                    a.counts[(size_t)g * a.stride + c] = v;
-            }
-        } else {
-            for (uint32_t g = threadIdx.x; g < a.M; g += blockDim.x) a.counts[(size_t)g * a.stride + c] = cnt[g];
+    __syncthreads();
+    if (NARROW) {
+        // After a wrap the column already holds the credited 65536s: add to it.
+        const bool add = wrapped != 0u;
+        for (uint32_t g = threadIdx.x; g < a.M; g += blockDim.x) {
+            const uint32_t v = (cnt[g >> 1] >> ((g & 1u) << 4)) & 0xFFFFu;
+            if (add)
+                atomicAdd(&a.counts[(size_t)g * a.stride + c], v);
+            else
+                a.counts[(size_t)g * a.stride + c] = v;
         }
+    } else {
+        for (uint32_t g = threadIdx.x; g < a.M; g += blockDim.x) a.counts[(size_t)g * a.stride + c] = cnt[g];
     }
 }
 
@@ -440,9 +419,9 @@ static size_t chunk_str_smem(uint64_t partitions, bool narrow) {
     return 4 * ((words + 3) & ~size_t(3)) + (size_t)(kChunkThreads / 32) * kStrStageBytes;
 }
 
-template <int KIND, bool SCATTER, bool NARROW>
+template <int KIND, bool NARROW>
 static cudaError_t launch_chunk(const MapArgs &a, const MapPlan &plan, cudaStream_t st) {
-    if constexpr (KIND == PHOBIC_KEYS_STRINGS && !SCATTER) {
+    if constexpr (KIND == PHOBIC_KEYS_STRINGS) {
         // Staged string loads whenever the stages fit beside the counters.
         const size_t smem = chunk_str_smem(a.M, NARROW);
         if (allow_dynamic_smem(k_chunk_str<NARROW>, smem) == cudaSuccess) {
@@ -452,20 +431,17 @@ static cudaError_t launch_chunk(const MapArgs &a, const MapPlan &plan, cudaStrea
         cudaGetLastError();
     }
     const size_t smem = chunk_smem(a.M, NARROW);
-    cudaError_t e = allow_dynamic_smem(k_chunk<KIND, SCATTER, NARROW>, smem);
+    cudaError_t e = allow_dynamic_smem(k_chunk<KIND, NARROW>, smem);
     if (e != cudaSuccess) return e;
-    k_chunk<KIND, SCATTER, NARROW><<<plan.grid, kChunkThreads, smem, st>>>(a);
+    k_chunk<KIND, NARROW><<<plan.grid, kChunkThreads, smem, st>>>(a);
     return cudaSuccess;
 }
 
 template <bool SCATTER, int KIND>
 static cudaError_t launch_kind(const MapArgs &a, const MapPlan &plan, cudaStream_t st) {
     if (plan.chunked) {
-        cudaError_t e;
-        if constexpr (SCATTER)
-            e = plan.narrow ? cudaErrorInvalidValue : launch_chunk<KIND, true, false>(a, plan, st);
-        else
-            e = plan.narrow ? launch_chunk<KIND, false, true>(a, plan, st) : launch_chunk<KIND, false, false>(a, plan, st);
+        if constexpr (SCATTER) return cudaErrorInvalidValue;
+        const cudaError_t e = plan.narrow ? launch_chunk<KIND, true>(a, plan, st) : launch_chunk<KIND, false>(a, plan, st);
         if (e != cudaSuccess) return e;
     } else {
         k_map<KIND, SCATTER><<<plan.grid, kMapThreads, 0, st>>>(a);
