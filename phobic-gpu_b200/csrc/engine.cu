@@ -394,6 +394,10 @@ phobic_status check_params(const phobic_params *params, uint32_t *cap, uint32_t 
     return PHOBIC_OK;
 }
 
+// The count matrix is read for the last time (K2) before the first record of K3 is written, so it lies
+// where the records come to lie, unless it is larger (partitions of a few keys).
+static bool counts_apart(uint64_t keys, uint64_t entries) { return 4 * entries > 16 * keys; }
+
 uint64_t sets_arena_bytes(const phobic_keys *sets, uint32_t nsets, const phobic_params *params,
                           const phobic_result *results, bool debug) {
     const uint64_t P = params->partition_size, B = params->buckets;
@@ -408,7 +412,8 @@ uint64_t sets_arena_bytes(const phobic_keys *sets, uint32_t nsets, const phobic_
     t += align256(4 * kFulcrums) + align256(sizeof(SetDesc) * nsets) + 2 * align256(8 * (nsets + 1)) +
          align256(8 * nsets);
     const uint64_t MS = M * plan_map(N, M, 0).stride;  // count matrix entries
-    t += align256(4 * MS) + align256(4 * (MS + 1)) + align256(64 + 8 * ((MS + kScanTile - 1) / kScanTile) + 8);
+    if (counts_apart(N, MS)) t += align256(4 * MS);
+    t += align256(4 * (M + 1)) + align256(64 + 8 * ((MS + kScanTile - 1) / kScanTile) + 8);
     if (nsets && sets[0].kind == PHOBIC_KEYS_STRINGS) t += align256(16 * N);
     // lowers, bucket ids, partition records (also the search's scratch), cursors
     t += align256(8 * N) + align256(2 * N) + align256(16 * N) + align256(4 * M) + align256(4 * kMaxBins);
@@ -559,8 +564,8 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
     uint32_t *d_fulcs = reinterpret_cast<uint32_t *>(d_tab + tab_desc + tab_kb + tab_pb);
     unsigned long long *d_err = reinterpret_cast<unsigned long long *>(d_tab + tab_in);
     const uint64_t MS = M * plan.stride;  // count matrix entries
-    uint32_t *d_count = static_cast<uint32_t *>(take(4 * MS));
-    uint32_t *d_G = static_cast<uint32_t *>(take(4 * (MS + 1)));
+    uint32_t *d_count = counts_apart(N, MS) ? static_cast<uint32_t *>(take(4 * MS)) : nullptr;
+    uint32_t *d_G = static_cast<uint32_t *>(take(4 * (M + 1)));
     const uint32_t tiles = (uint32_t)((MS + kScanTile - 1) / kScanTile);
     // What a build finds at zero, side by side: the search's queue, the scan's tiles and tile counter.
     const size_t zero_bytes = 64 + 8 * (size_t)tiles + 8;
@@ -571,6 +576,7 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
     uint16_t *d_bkt = static_cast<uint16_t *>(take(2 * N));
     uint4 *d_inter = static_cast<uint4 *>(take(16 * N));
     uint2 *d_sorted = reinterpret_cast<uint2 *>(d_inter);  // K3c, after K3b is done with d_inter
+    if (!d_count) d_count = reinterpret_cast<uint32_t *>(d_inter);
     uint32_t *d_pcur = static_cast<uint32_t *>(take(4 * M));
     uint32_t *d_bincur = static_cast<uint32_t *>(take(4 * kMaxBins));
     uint4 *d_dbg_keys = debug ? static_cast<uint4 *>(take(16 * N)) : nullptr;
@@ -586,13 +592,13 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
     const SearchShape shape = choose_search_shape(w, params, (uint32_t)M);
     MapArgs ma{d_desc, d_kb, nsets, B, N, d_fulcs, d_count, d_mapped, d_dbg_keys, d_lowers, d_bkt, d_err,
                (uint32_t)M, plan.stride, plan.chunk};
-    ScanArgs sa{d_count, d_G, nullptr, (uint32_t)MS, d_tiles, reinterpret_cast<uint32_t *>(d_tiles + tiles), nsets,
-                d_err, 0, d_pcur, d_bincur, plan.stride, wshift};
+    ScanArgs sa{d_count, d_G, d_pcur, (uint32_t)MS, d_tiles, reinterpret_cast<uint32_t *>(d_tiles + tiles), nsets,
+                d_err, 0, plan.stride, d_bincur, wshift};
     PartArgs pa{d_inter, d_bincur, d_pcur, wshift, (uint32_t)((M + (1ull << wshift) - 1) >> wshift), (uint32_t)M};
     // (The injected change needs two readers of the keys: with one partition, K1 and K3.)
     const bool small = nsets == 1 && !debug && !(key_change && M < 2) && gather_fits(kind, N, M, B, cap);
-    SearchArgs qa{d_desc, d_pb, nsets, (uint32_t)M, d_G, small ? 1u : plan.stride, d_lowers, d_bkt, d_sorted, d_dbg_sizes, B, cap,
-                  k_max, d_queue, d_err, d_pcur, P};
+    SearchArgs qa{d_desc, d_pb, nsets, (uint32_t)M, d_G, d_lowers, d_bkt, d_sorted, d_dbg_sizes, B, cap, k_max, d_queue,
+                  d_err, d_pcur, P};
 
     // The device stages, from the per-build memsets to the status copy: enqueued one by one,
     // or under stream capture (the stage events then become event-record nodes of the graph).
@@ -605,7 +611,7 @@ phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, c
             PHB_TRY(record(w.ev[1]), "event");
             {
                 StageRange r("bucket_sizes, partition_offsets, key_redistribution (K1-K3)");
-                PHB_TRY(launch_gather(kind, ma, qa, d_G, d_count, d_queue + 8, s, kc_index, key_change ? kc_mask : 0),
+                PHB_TRY(launch_gather(kind, ma, qa, d_G, d_bincur, d_queue + 8, s, kc_index, key_change ? kc_mask : 0),
                         "gather");
             }
             if (key_change)

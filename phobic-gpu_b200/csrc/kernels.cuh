@@ -20,13 +20,16 @@ namespace phobicb200 {
 constexpr int kMapThreads = 256;
 // Chunked counting: CTA c owns the keys [c * chunk, (c + 1) * chunk) and keeps a
 // counter for every partition in shared memory; the count matrix is stored
-// partition-major (entry g * stride + c, stride = number of chunks), so its
-// exclusive scan gives each chunk its own slot range inside every partition.
+// partition-major (entry g * stride + c, stride = number of chunks), so that its
+// exclusive scan passes every partition's offset.
 constexpr int kChunkThreads = 1024;
 constexpr uint32_t kChunkCtas = 148;                 // one CTA per SM of a B200
 // Smallest chunk worth a CTA, two keys a thread: against 16,384 keys the counting of 700,001 strings
-// takes 25 us, not 60, of 10^6 u64 keys 11, not 15.
+// takes 25 us, not 60, of 10^6 u64 keys 11, not 15.  Only while the count matrix holds no more entries than there
+// are keys (or chunks of kChunkKeys give as many): 300,000 keys in partitions of 32 would have 147 columns, not
+// 32, and 4 MB of the scan's input, not 1; counting and scan took 45 us so, and take 33.
 constexpr uint64_t kChunkMinKeys = 2048;
+constexpr uint64_t kChunkKeys = 16384;
 constexpr uint32_t kChunkMaxPartitions = 52 * 1024;  // 32-bit shared-memory counters per CTA
 // Counting only (K1): above kChunkMaxPartitions the counters are packed two to a
 // 32-bit word.  A 16-bit counter that wraps is caught from the atomic's return value
@@ -115,18 +118,18 @@ uint32_t part_wshift(uint64_t partitions);
 
 struct ScanArgs {
     const uint32_t *in;              // [m] count matrix, partition-major
-    uint32_t *out;                   // [m + 1] exclusive prefix, out[m] = total
-    uint32_t *cursor;                // [m] copy of out[0..m) (global-counter scatter cursors) or null
+    uint32_t *out;                   // [m / stride + 1] offset of every partition (entry g * stride), then the total
+    uint32_t *cursor;                // [m / stride] copy of out less the total: placement cursors (may be `in` for stride 1)
     uint32_t m;                      // partitions * stride
     unsigned long long *tile_state;  // [tiles], zeroed: (flag << 32) | value
     uint32_t *tile_counter;          // zeroed
     uint32_t nsets;
     unsigned long long *err;         // [nsets]
     unsigned long long wait_ns;      // bound of the look-back wait on a predecessor tile
-    // Two-pass partition (or null): offset of every partition (entry g * stride) and of every
-    // coarse bin's first partition.
-    uint32_t *pcur = nullptr, *bincur = nullptr;
-    uint32_t stride = 1, wshift = 0;
+    uint32_t stride = 1;
+    // Two-pass partition (or null): offset of every coarse bin's first partition.
+    uint32_t *bincur = nullptr;
+    uint32_t wshift = 0;
 };
 
 struct SearchArgs {
@@ -134,10 +137,9 @@ struct SearchArgs {
     const uint32_t *part_base;  // [nsets + 1]
     uint32_t nsets;
     uint32_t M;                 // global partitions
-    const uint32_t *G;          // [M * gstride + 1] record offsets; partition g spans [G[g*gstride], G[(g+1)*gstride])
-    uint32_t gstride;
+    const uint32_t *G;          // [M + 1] record offsets; partition g spans [G[g], G[g + 1])
     // Partition-contiguous records; K3c leaves a partition's search schedule in the place of its
-    // lower pairs (words 2 * G[g * gstride] ...).
+    // lower pairs (words 2 * G[g] ...).
     const uint2 *lowers;
     const uint16_t *bkt;
     uint2 *sorted;              // lower pairs in search order, same indexing as lowers
@@ -225,11 +227,12 @@ size_t search_group_smem(uint32_t buckets, uint32_t cap, int W);
 unsigned int check_line_map(bool reset);
 unsigned int check_line_part(bool reset);
 // Small builds of one set of fixed-size keys: K1, the scan and K3 in one launch (kernels_order.cu).
-// gather_fits says whether a build is one; G [M + 1] gets the partition offsets (stride 1), ends [M]
+// gather_fits says whether a build is one; G [M + 1] gets the partition offsets, ends [M]
 // is scratch, ticket [4] (8-byte aligned) starts at zero.  change_mask (tests; u64 keys) stands for a
 // key that is written while the CTAs read: all but the first see key change_index changed by it.
 constexpr uint64_t kGatherMaxKeys = 12288;
 constexpr uint64_t kGatherMaxPartitions = 148;  // one CTA per SM
+static_assert(kGatherMaxPartitions <= kMaxBins, "the ends lie in the bin cursors' array");
 bool gather_fits(int kind, uint64_t n, uint64_t M, uint32_t B, uint32_t cap);
 cudaError_t launch_gather(int kind, const MapArgs &m, const SearchArgs &a, uint32_t *G, uint32_t *ends, uint32_t *ticket,
                           cudaStream_t st, uint64_t change_index = 0, uint64_t change_mask = 0);

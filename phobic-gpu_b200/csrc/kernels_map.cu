@@ -395,7 +395,10 @@ static size_t chunk_smem(uint64_t partitions, bool narrow) {
 MapPlan plan_map(uint64_t total_keys, uint64_t partitions, int sm_count) {
     MapPlan p{};
     if (partitions <= kChunkNarrowMaxPartitions && total_keys > 0) {
-        uint64_t ctas = (total_keys + kChunkMinKeys - 1) / kChunkMinKeys;
+        const uint64_t fine = (total_keys + kChunkMinKeys - 1) / kChunkMinKeys,
+                       coarse = (total_keys + kChunkKeys - 1) / kChunkKeys;
+        uint64_t ctas = fine * partitions <= total_keys ? fine : total_keys / (partitions ? partitions : 1);
+        if (ctas < coarse) ctas = coarse;
         if (ctas > kChunkCtas) ctas = kChunkCtas;
         p.chunked = true;
         p.stride = (uint32_t)ctas;

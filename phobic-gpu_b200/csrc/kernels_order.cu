@@ -225,7 +225,7 @@ __global__ void __launch_bounds__(kOrderThreads, kOrderCtas) k_order(SearchArgs 
         const uint32_t s_idx = a.nsets == 1 ? 0u : find_set(a.part_base, a.nsets, g);
         const SetDesc &d = a.sets[s_idx];
         const uint32_t p = g - d.part_base;
-        const uint32_t base = a.G[(size_t)g * a.gstride], end = a.G[(size_t)(g + 1) * a.gstride];
+        const uint32_t base = a.G[g], end = a.G[g + 1];
         const uint32_t ps = end - base;
         // The size check comes first and looks at every partition, also of a set that failed before
         // (only a scan that timed out leaves no offsets to check): the error word then holds the
@@ -241,11 +241,11 @@ __global__ void __launch_bounds__(kOrderThreads, kOrderCtas) k_order(SearchArgs 
             state = kPartSkipped;
         } else {
             if (d.part_off) {
-                const uint32_t g0 = a.G[(size_t)d.part_base * a.gstride];
+                const uint32_t g0 = a.G[d.part_base];
                 d.part_off[p] = base - g0;
                 if (p + 1 == d.partitions) d.part_off[p + 1] = end - g0;
             }
-            if (!PHB_CHECK(base + ps <= a.G[(size_t)a.M * a.gstride])) {
+            if (!PHB_CHECK(base + ps <= a.G[a.M])) {
                 state = kPartSkipped;
             } else if (a.part_state[g] != end) {
                 // K3 placed exactly the keys K1 counted, unless the keys changed in between.

@@ -6,8 +6,8 @@
 // (include/phobicGpu/mphf_builder.h:254-257): out[0] = 0, out[p + 1] = out[p] + size[p].
 // The scanned array is the (partition, chunk) count matrix of K1, so the prefix
 // is at once every partition's record offset and every chunk's scatter cursor.
-// The tile that holds a partition's first entry also seeds its placement cursor and, for a
-// coarse bin's first partition, the bin's.
+// Only the prefix at a partition's first entry is kept: the tile that holds it writes the
+// partition's offset and its placement cursor and, for a coarse bin's first partition, the bin's.
 //
 // Each CTA takes the next tile id from a counter, so every tile it waits on was
 // started before it; the wait on a predecessor is still bounded in time
@@ -94,24 +94,21 @@ __global__ void __launch_bounds__(kScanThreads) k_scan(ScanArgs a) {
     uint32_t run = s_prefix + s_warp[warp] + incl - sum;
     // The next partition that starts at or after this thread's first entry.
     const uint32_t b32 = (uint32_t)base;  // entries number less than 2^32
-    uint64_t g = a.pcur && base < a.m ? b32 / a.stride + (b32 % a.stride != 0) : 0, first = g * a.stride;
+    uint64_t g = base < a.m ? b32 / a.stride + (b32 % a.stride != 0) : 0, first = g * a.stride;
 #pragma unroll
     for (int j = 0; j < kScanItems; j++) {
         uint64_t idx = base + j;
-        if (idx < a.m) {
-            a.out[idx] = run;
-            if (a.cursor) a.cursor[idx] = run;
-            if (a.pcur && idx == first) {
-                a.pcur[g] = run;
-                if ((g & ((1ull << a.wshift) - 1)) == 0) a.bincur[g >> a.wshift] = run;
-                g++;
-                first += a.stride;
-            }
+        if (idx < a.m && idx == first) {
+            a.out[g] = run;
+            if (a.cursor) a.cursor[g] = run;
+            if (a.bincur && (g & ((1ull << a.wshift) - 1)) == 0) a.bincur[g >> a.wshift] = run;
+            g++;
+            first += a.stride;
         }
         run += v[j];
     }
     // The thread holding the last element also writes the total.
-    if (base <= (uint64_t)a.m - 1 && (uint64_t)a.m - 1 < base + kScanItems) a.out[a.m] = run;
+    if (base <= (uint64_t)a.m - 1 && (uint64_t)a.m - 1 < base + kScanItems) a.out[a.m / a.stride] = run;
 }
 
 cudaError_t launch_scan(const ScanArgs &a, cudaStream_t st) {

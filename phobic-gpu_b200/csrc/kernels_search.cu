@@ -676,8 +676,8 @@ __device__ __forceinline__ uint32_t search_partition(const SearchArgs &a, uint32
                                                      const SetDesc &d, uint32_t g, uint32_t p, int lane) {
     const uint32_t nonempty = a.part_state[g];
     if (nonempty & kPartSkipped) return nonempty & ~kPartSkipped;
-    const uint32_t base = a.G[(size_t)g * a.gstride];
-    const uint32_t ps = a.G[(size_t)(g + 1) * a.gstride] - base;
+    const uint32_t base = a.G[g];
+    const uint32_t ps = a.G[g + 1] - base;
     if (ps == 0) return PHOBIC_OK;
     load_partition(a, w, ws, base, ps, nonempty, (uint32_t)lane, 32);
     __syncwarp();
@@ -1012,8 +1012,8 @@ __global__ void __launch_bounds__(kSearchWarps * 32, 2) k_search_group(SearchArg
         group_bar(bar_id, bar_n);
         const uint32_t nonempty = ctl[1];
         if (nonempty != 0xFFFFFFFFu) {
-            const uint32_t base = a.G[(size_t)g * a.gstride];
-            const uint32_t ps = a.G[(size_t)(g + 1) * a.gstride] - base;
+            const uint32_t base = a.G[g];
+            const uint32_t ps = a.G[g + 1] - base;
             const uint2 *so = a.sorted + base;
             uint32_t *pil = d.pilots + p;
             const size_t pstride = d.partitions;

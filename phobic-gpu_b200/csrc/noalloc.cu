@@ -174,7 +174,7 @@ extern "C" phobic_status phobic_build_noalloc(const phobic_keys *keys, const pho
                    (uint32_t)m, 1, 0};
         ScanArgs sa{d_count, d_G, d_count, (uint32_t)m, d_tiles, reinterpret_cast<uint32_t *>(d_tiles + tiles), 1,
                     d_err, 0};
-        SearchArgs qa{d_desc, d_pb, 1, (uint32_t)m, d_G, 1, d_lowers, d_bkt, d_sorted, nullptr, B, cap, k_max,
+        SearchArgs qa{d_desc, d_pb, 1, (uint32_t)m, d_G, d_lowers, d_bkt, d_sorted, nullptr, B, cap, k_max,
                       d_queue, d_err, d_count, P};
         uint64_t kc_index = 0, kc_mask = 0;
         ok = cuda(launch_map_count(keys->kind, ma, plan, s));

@@ -158,3 +158,15 @@ def test_accepted_bucket_counts_follow_the_documented_rule(phobic, cap):
     top = max(B for B in range(1, 65_536) if 4 * words(B) <= 227 * 1024)
     for B in (1, 512, 513, top - 1, top, top + 1, 65_535):
         assert accepted(B) == (4 * words(B) <= 227 * 1024), B
+
+
+@pytest.mark.parametrize("P,n", [(8, 100_000), (8, 300_000), (32, 300_000), (64, 1_000_000), (256, 300_000),
+                                 (2048, 700_001), (2048, 1_000_000), (2500, 2_000_000), (64, 40_000_000)])
+def test_count_matrix_of_small_partitions_stays_small(phobic, P, n):
+    """Device bytes of a build: 26 bytes a key (records), the results, tables per partition, and for the
+    counts no more than 8 bytes per partition and chunk of 16,384 keys (at most 148 chunks)."""
+    cfg = phobic.MPHFconfig(5.0, P)
+    M, B = cfg.partitions(n), cfg.bucketCountPerPartition
+    keys = phobic.Keys(phobic.KEYS_U64, 1, n, 4096, None)
+    need = phobic.lib().phobic_build_bytes_needed(C.byref(keys), C.byref(cfg.params))
+    assert 26 * n < need <= 26 * n + 8 * M * min(148, -(-n // 16_384)) + 4 * B * M + 24 * M + 32_768
