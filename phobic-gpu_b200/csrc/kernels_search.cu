@@ -865,6 +865,13 @@ __device__ __forceinline__ uint32_t ksplit_bucket(const WarpSmem &ws, const uint
     }
 }
 
+// Offsets of a bucket's windows that are taken on its turn before the windows are read again (one
+// look at the slots and one reduction each; reading them anew takes about three times as long).  In
+// partitions of few slots nearly all offsets of the first buckets' windows are gone by their turn: with the windows
+// walked to their end the search of 1000 keys takes 189 us at P 256 and 177 at P 128, with 8, 4, 2 and 1
+// steps 52, 46, 40 and 36 at P 256; at P 2048, where steps are few, 1 and 2 are up to 4 % slower than 4.
+constexpr uint32_t kStaleSteps = 4;
+
 // The bucket pipeline of a group from bucket `first` on (see k_search_group); NR as in
 // seek_batched.
 template <int W, int NR>
@@ -914,6 +921,7 @@ __device__ __forceinline__ void pipeline(const WarpSmem &ws, const uint2 *so, co
         // One lane reads the status, which another warp may be writing: the warp agrees on what it saw.
         uint32_t st = __shfl_sync(kFullMask, lane == 0 ? *status : 0u, 0), q = 0, at = 0, bit = 0;
         bool turn = false, seek = st == PHOBIC_OK, on = false;
+        uint32_t gone = 0;
 #pragma unroll 1
         for (;;) {
             if (seek) st = seek_any<NR>(ws, ws.hs + half, L, s, sr, fm, k_lim, lane, &f);
@@ -928,16 +936,18 @@ __device__ __forceinline__ void pipeline(const WarpSmem &ws, const uint2 *so, co
                 turn = true;
             }
             if (!__any_sync(kFullMask, lds32(at) & bit)) break;
-            // An earlier bucket took a slot since: the next free offset of the same windows, or
-            // the next counter.
+            // An earlier bucket took a slot since: the next free offset of the same windows or, when
+            // a few of them were gone too, of the windows as they are now, or the next counter.
             seek = true;
             if constexpr (NR > 0) {
+                if (++gone % kStaleSteps != 0) {
 #pragma unroll
-                for (int r = 0; r < NR; r++)
-                    if (f.o >> 5 == (uint32_t)(32 * r + lane)) f.bad[r] |= 1u << (f.o & 31);
-                f.o = smallest_offset<NR>(f.bad, lane);
-                seek = f.o == kNone;
-                if (seek) ++f.k;
+                    for (int r = 0; r < NR; r++)
+                        if (f.o >> 5 == (uint32_t)(32 * r + lane)) f.bad[r] |= 1u << (f.o & 31);
+                    f.o = smallest_offset<NR>(f.bad, lane);
+                    seek = f.o == kNone;
+                    if (seek) ++f.k;
+                }
             }
         }
         mark_own(at, bit, on);

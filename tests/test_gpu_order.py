@@ -89,3 +89,18 @@ def test_small_builds_report_errors_like_the_oracle(phobic):
             assert e.value.status == want
         got = ctx.build(keys, cfg)
         assert (got.pilots == O.build(O.hash_keys(keys, "u64"), 2048, cfg.bucketCountPerPartition, cfg.getFulcs())["pilots"]).all()
+
+
+@pytest.mark.parametrize("group,pipe", [(1, 0), (4, 0), (2, 1), (4, 1), (8, 1), (0, 0)])
+@pytest.mark.parametrize("P,n", [(16, 20), (32, 200), (64, 9_000), (128, 30_000), (256, 1_000), (300, 40_000), (512, 90_000)])
+def test_small_partitions_match_oracle(phobic, P, n, group, pipe):
+    """Partitions of few slots: most offsets of a bucket's windows are gone by its turn, most of its
+    pilot counters put two keys on one slot, and a partition is ordered by one warp."""
+    cfg = phobic.MPHFconfig(5.0, P)
+    keys = keygen.splitmix64(8000 + P, n)
+    want = O.build(O.hash_keys(keys, "u64"), P, cfg.bucketCountPerPartition, cfg.getFulcs())
+    assert want["status"] == 0
+    with phobic.Context(0) as ctx:
+        ctx.set_tuning(search_group=group, search_pipeline=pipe)
+        got = ctx.build(keys, cfg)
+    assert (got.pilots == want["pilots"]).all() and (got.partition_offsets == want["offsets"]).all()
