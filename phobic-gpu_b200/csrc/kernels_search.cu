@@ -477,14 +477,24 @@ __device__ __forceinline__ uint32_t seek_any(const WarpSmem &ws, uint32_t *hs, u
 
 // One bucket of more than 32 keys (a few per partition).  Each try hashes chunk by chunk and
 // stops at the first chunk that repeats a slot: buckets of 100 to 160 keys are rejected about 37
-// times per partition (10^8 u64 keys, lambda 7, P 2500), after 62 keys on average.  The keys are
-// read from the bucket-ordered copy on every try: staging them in shared memory takes that much
+// times per partition (10^8 u64 keys, lambda 7, P 2500), after 62 keys on average.  In partitions of few
+// slots nearly every try ends at the first chunk, after thousands of tries in the worst of them, and the
+// build lasts as long as those take: the first chunk's keys are in registers, and its slots under
+// the next counter are formed while this counter's are tested.  The other keys are read
+// from the bucket-ordered copy on every try: staging them in shared memory takes that much
 // from the L1 that the copy and the schedule are read through, and was slower (search 6.18
 // against 6.06 ms).
 __device__ __forceinline__ uint32_t place_large(const WarpSmem &ws, const uint2 *src, uint32_t s, const ScanRange &sr,
                                                 FastMod fm, uint32_t k_lim, int lane, uint32_t *pilot) {
     const uint32_t padded = (s + 3) & ~3u, ps = sr.ps;
     const uint32_t hs_sa = (uint32_t)__cvta_generic_to_shared(ws.hs);
+    // The collision test of one key (its bit in the warp's scratch, clear before).
+    auto taken = [&](uint32_t h) {
+        const uint32_t bit = 1u << (h & 31);
+        return PHB_CHECK(h < ps) && (atomicOr(&ws.scr[h >> 5], bit) & bit) != 0;
+    };
+    const uint2 key0 = src[lane];
+    uint32_t h_next = fm.mod(pilot_hash(key0.x, key0.y, 0u));
     for (uint32_t k = 0; k < k_lim; k++) {
         if (k == kDupCheckAt) {
             bool d = false;
@@ -494,17 +504,25 @@ __device__ __forceinline__ uint32_t place_large(const WarpSmem &ws, const uint2 
             }
             if (__any_sync(kFullMask, d)) return PHOBIC_ERR_DUPLICATE_KEY;
         }
+        const uint32_t h0 = h_next;
+        const bool d0 = taken(h0);
+        h_next = fm.mod(pilot_hash(key0.x, key0.y, k + 1));
+        if (__any_sync(kFullMask, d0)) {
+            if (PHB_CHECK(h0 < ps)) ws.scr[h0 >> 5] = 0;
+            __syncwarp();
+            continue;
+        }
+        ws.hs[lane] = pack_slot(h0);
         bool dup = false;
-        uint32_t done = 0;  // keys hashed (and marked in the collision scratch)
-        for (uint32_t c0 = 0; c0 < s && !dup; c0 += 32) {
+        uint32_t done = 32;  // keys hashed (and marked in the collision scratch)
+        for (uint32_t c0 = 32; c0 < s && !dup; c0 += 32) {
             const uint32_t i = c0 + lane;
             bool d = false;
             if (i < s) {
                 const uint2 key = src[i];
                 const uint32_t h = fm.mod(pilot_hash(key.x, key.y, k));
                 ws.hs[i] = pack_slot(h);
-                const uint32_t bit = 1u << (h & 31);
-                d = PHB_CHECK(h < ps) && (atomicOr(&ws.scr[h >> 5], bit) & bit) != 0;
+                d = taken(h);
             }
             dup = __any_sync(kFullMask, d);
             done = c0 + 32;

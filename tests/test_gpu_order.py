@@ -104,3 +104,23 @@ def test_small_partitions_match_oracle(phobic, P, n, group, pipe):
         ctx.set_tuning(search_group=group, search_pipeline=pipe)
         got = ctx.build(keys, cfg)
     assert (got.pilots == want["pilots"]).all() and (got.partition_offsets == want["offsets"]).all()
+
+
+def test_crowded_buckets_match_oracle(phobic):
+    """Large buckets that nearly always meet themselves: the first chunk of 32 keys ends most tries, the second
+    one some, in the one-warp search of partitions of few slots (128 and fewer) and of more."""
+    for lam, P, n in ((8.0, 100, 2_000), (7.0, 64, 640), (6.0, 160, 8_000), (10.0, 700, 14_000), (10.0, 160, 8_000)):
+        cfg = phobic.MPHFconfig(lam, P)
+        keys = keygen.splitmix64(8100 + P, n)
+        want = O.build(O.hash_keys(keys, "u64"), P, cfg.bucketCountPerPartition, cfg.getFulcs(), max_k=20_000)
+        cfg.params.max_pilot_counter = 20_000
+        with phobic.Context(0) as ctx:
+            for group, pipe in ((1, 0), (8, 1)):
+                ctx.set_tuning(search_group=group, search_pipeline=pipe)
+                if want["status"] != 0:
+                    with pytest.raises(phobic.PhobicError) as e:
+                        ctx.build(keys, cfg)
+                    assert e.value.status == want["status"]
+                    continue
+                got = ctx.build(keys, cfg)
+                assert (got.pilots == want["pilots"]).all() and (got.partition_offsets == want["offsets"]).all()
