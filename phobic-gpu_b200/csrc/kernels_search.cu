@@ -35,6 +35,7 @@
 // loads).  Larger buckets read their keys from the bucket-ordered copy in global
 // memory.
 #include <algorithm>
+#include <type_traits>
 
 #include "kernels.cuh"
 
@@ -177,11 +178,15 @@ __device__ __forceinline__ bool round_result(uint32_t bad, uint32_t o0, uint32_t
 // Round R of a block of three: the windows of a bucket of at most S = 4 or 8 keys whose packed
 // slots are in v and whose pair addresses (this lane's window offset included) are in a.  The
 // last two keys of S are skipped when the bucket is that small.
-template <int S, int R>
+// DENSE: no further keys once the first four have closed every lane's window.
+template <int S, int R, bool DENSE = false>
 __device__ __forceinline__ uint32_t round_bad(const WarpSmem &ws, const uint32_t (&a)[S], const uint32_t (&v)[S],
                                               bool full, uint32_t bad) {
 #pragma unroll
-    for (int i = 0; i < S - 2; i++) bad |= window_at<256 * R>(ws, a[i], v[i]);
+    for (int i = 0; i < S - 2; i++) {
+        if (DENSE && i == 4 && __all_sync(kFullMask, bad == kFullMask)) return bad;
+        bad |= window_at<256 * R>(ws, a[i], v[i]);
+    }
     if (full) bad |= window_at<256 * R>(ws, a[S - 2], v[S - 2]) | window_at<256 * R>(ws, a[S - 1], v[S - 1]);
     return bad;
 }
@@ -192,7 +197,7 @@ __device__ __forceinline__ uint32_t round_bad(const WarpSmem &ws, const uint32_t
 // inside the padded bitmap (bitmap_pairs) and are masked.
 // The masks of the rounds are held per partition: chosen in every round, with the loop over blocks
 // of rounds below for every partition, the search of 10^8 u64 keys takes 5.49 instead of 5.36 ms.
-template <int S>
+template <int S, bool DENSE = false>
 __device__ __forceinline__ uint32_t scan_small(const WarpSmem &ws, uint32_t hs, uint32_t s, const ScanRange &sr,
                                                int lane) {
     const uint32_t lane_sa = ws.occ + 8u * lane;
@@ -206,11 +211,11 @@ __device__ __forceinline__ uint32_t scan_small(const WarpSmem &ws, uint32_t hs, 
     for (int i = 0; i < S; i++) a[i] = lane_sa + (v[i] >> 5);
     const bool full = s > S - 2;
     uint32_t o;
-    if (round_result(round_bad<S, 0>(ws, a, v, full, sr.dead0), 0, &o)) return o;
+    if (round_result(round_bad<S, 0, DENSE>(ws, a, v, full, sr.dead0), 0, &o)) return o;
     if (sr.rounds == 1) return kNone;
-    if (round_result(round_bad<S, 1>(ws, a, v, full, sr.dead1), 1024, &o)) return o;
+    if (round_result(round_bad<S, 1, DENSE>(ws, a, v, full, sr.dead1), 1024, &o)) return o;
     if (sr.rounds == 2) return kNone;
-    return round_result(round_bad<S, 2>(ws, a, v, full, sr.last_dead), 2048, &o) ? o : kNone;
+    return round_result(round_bad<S, 2, DENSE>(ws, a, v, full, sr.last_dead), 2048, &o) ? o : kNone;
 }
 
 // The same for a partition of more than three rounds: three at a time (scan_quads, which forms the
@@ -245,6 +250,7 @@ __device__ __forceinline__ uint32_t scan_blocks(const WarpSmem &ws, uint32_t hs,
 
 // The same for a bucket of any size: s packed slots at the shared address hs, padded to a
 // multiple of 4 with copies of one of them.
+template <bool DENSE = false>
 __device__ __forceinline__ uint32_t scan_quads(const WarpSmem &ws, uint32_t hs, uint32_t s, const ScanRange &sr,
                                                int lane) {
     uint32_t lane_sa = ws.occ + 8u * lane, o;
@@ -256,6 +262,7 @@ __device__ __forceinline__ uint32_t scan_quads(const WarpSmem &ws, uint32_t hs, 
             const uint4 v = lds128(q);
             bad |= window_at<0>(ws, lane_sa + (v.x >> 5), v.x) | window_at<0>(ws, lane_sa + (v.y >> 5), v.y);
             bad |= window_at<0>(ws, lane_sa + (v.z >> 5), v.z) | window_at<0>(ws, lane_sa + (v.w >> 5), v.w);
+            if (DENSE && __all_sync(kFullMask, bad == kFullMask)) break;
         }
         if (round_result(bad, 1024 * (r - 1), &o)) return o;
         if (r == sr.rounds) return kNone;
@@ -309,6 +316,15 @@ __device__ __forceinline__ bool slots_distinct(uint32_t *scr, uint32_t q, bool o
     return !hit;
 }
 
+// Builds of at most this many keys per partition are searched by the DENSE kernel: their partitions
+// need many counters, so what a failing one takes counts.  Search of 2*10^7 keys at P 128 19.9 ms without
+// it, 12.8 with it; at P 256 3.2 and 3.7.
+constexpr uint32_t kDenseSlots = 128;
+// Slots below which a bucket of S / 2 to S keys meets itself on so many pilot counters (half of them, at
+// about three quarters of S keys) that the test comes before the scan: search of 10^6 keys at P 32 77.8 ms
+// without, 49.1 with it, and 59.5 and 49.0 with limits of S * S and S * S / 4.
+constexpr uint32_t crowded(uint32_t S) { return S * S / 2; }
+
 // Lanes per pilot counter for a bucket of s <= 32 keys: 4, 8, 16 or 32.
 __device__ __forceinline__ uint32_t counter_lanes(uint32_t s) { return s <= 4 ? 4u : s <= 8 ? 8u : s <= 16 ? 16u : 32u; }
 // The key that lane `lane` loads of a bucket of s <= 32 keys: lane t * S + i takes key i, lanes
@@ -318,35 +334,54 @@ __device__ __forceinline__ uint32_t lane_key(uint32_t s, int lane) {
     return i < s ? i : 0u;
 }
 
+// The lanes whose packed slot is this lane's, among the keys of a bucket of s <= S keys under the same
+// counter (lane t * S + i: key i, counter t).
+template <int S>
+__device__ __forceinline__ uint32_t same_slot_lanes(uint32_t hk, uint32_t s, int lane) {
+    // Packed slots have 20 bits; lanes past the bucket take values of their own.
+    const bool key = ((uint32_t)lane & (S - 1u)) < s;
+    return __match_any_sync(kFullMask, key ? hk | ((uint32_t)lane / S) << 24 : 0x80000000u | (uint32_t)lane);
+}
+
 // A bucket of at most S keys (S = 4, 8, 16 or 32; more than S / 2 of them, or S = 4), L as
 // lane_key loads it.  The warp hashes 32 / S pilot counters at once (lane t * S + i holds key i
 // under counter k0 + t) into hs and tests them in counter order, so a counter that fails costs
 // no new hash.  Same result as trying k = 0, 1, 2, ... one at a time (search.comp:105-124).
-// SMALL: the partition has at most three rounds.
-template <int S, bool SMALL>
+// SMALL: the partition has at most three rounds.  DENSE: of few slots (kDenseSlots).  MEET: the counters
+// of a batch that put two keys on one slot are found by one match of all slots and not scanned.
+template <int S, bool SMALL, bool DENSE = false, bool MEET = false>
 __device__ __forceinline__ uint32_t place_batched(const WarpSmem &ws, uint2 L, uint32_t s, const ScanRange &sr,
                                                   FastMod fm, uint32_t k_lim, int lane, uint32_t *pilot) {
     constexpr uint32_t G = 32 / S;
     const uint32_t hs_sa = (uint32_t)__cvta_generic_to_shared(ws.hs);
     const bool mine = lane < (int)s;
     uint32_t stop = min(k_lim, kDupCheckAt);  // a multiple of G, or k_lim
+    uint32_t hk_next = MEET ? pack_slot(fm.mod(pilot_hash(L.x, L.y, (uint32_t)lane / S))) : 0u;
     for (uint32_t k0 = 0;; k0 += G) {
         if (k0 >= stop) {
             if (k0 >= k_lim) return PHOBIC_ERR_SEARCH_LIMIT;
             if (s > 1 && has_duplicate_key(L, s, lane)) return PHOBIC_ERR_DUPLICATE_KEY;
             stop = k_lim;
         }
-        const uint32_t hk = pack_slot(fm.mod(pilot_hash(L.x, L.y, k0 + (uint32_t)lane / S)));
+        const uint32_t hk = MEET ? hk_next : pack_slot(fm.mod(pilot_hash(L.x, L.y, k0 + (uint32_t)lane / S)));
+        uint32_t meet = 0;  // lanes whose slot is that of another key under their counter
+        if constexpr (MEET) {
+            const uint32_t same = same_slot_lanes<S>(hk, s, lane);
+            hk_next = pack_slot(fm.mod(pilot_hash(L.x, L.y, k0 + G + (uint32_t)lane / S)));  // during the match
+            meet = __ballot_sync(kFullMask, (same & (same - 1u)) != 0u);
+            if (G == 1 && meet) continue;
+        }
         __syncwarp();
         ws.hs[lane] = hk;
         __syncwarp();
         const uint32_t tries = min(G, k_lim - k0);
 #pragma unroll 1
         for (uint32_t u = 0; u < tries; u++) {
+            if (MEET && (meet >> (S * u)) & (kFullMask >> (32 - S))) continue;
             uint32_t o;
-            if constexpr (S <= 8 && SMALL) o = scan_small<S>(ws, hs_sa + 4 * S * u, s, sr, lane);
+            if constexpr (S <= 8 && SMALL) o = scan_small<S, DENSE>(ws, hs_sa + 4 * S * u, s, sr, lane);
             else if constexpr (S <= 8) o = scan_blocks<S>(ws, hs_sa + 4 * S * u, s, sr, lane);
-            else o = scan_quads(ws, hs_sa + 4 * S * u, s, sr, lane);
+            else o = scan_quads<DENSE>(ws, hs_sa + 4 * S * u, s, sr, lane);
             if (o == kNone) continue;
             uint32_t q = unpack_slot(ws.hs[S * u + (mine ? (uint32_t)lane : 0u)]) + o;
             q = q >= sr.ps ? q - sr.ps : q;
@@ -484,6 +519,7 @@ __device__ __forceinline__ uint32_t seek_any(const WarpSmem &ws, uint32_t *hs, u
 // from the bucket-ordered copy on every try: staging them in shared memory takes that much
 // from the L1 that the copy and the schedule are read through, and was slower (search 6.18
 // against 6.06 ms).
+template <bool DENSE>
 __device__ __forceinline__ uint32_t place_large(const WarpSmem &ws, const uint2 *src, uint32_t s, const ScanRange &sr,
                                                 FastMod fm, uint32_t k_lim, int lane, uint32_t *pilot) {
     const uint32_t padded = (s + 3) & ~3u, ps = sr.ps;
@@ -532,7 +568,7 @@ __device__ __forceinline__ uint32_t place_large(const WarpSmem &ws, const uint2 
         if (dup) continue;
         if (s + lane < padded) ws.hs[s + lane] = ws.hs[0];
         __syncwarp();
-        const uint32_t o = scan_quads(ws, hs_sa, s, sr, lane);
+        const uint32_t o = scan_quads<DENSE>(ws, hs_sa, s, sr, lane);
         __syncwarp();
         if (o == kNone) continue;
         for (uint32_t i = lane; i < s; i += 32) {
@@ -669,7 +705,7 @@ __device__ __forceinline__ void advance(const WarpSmem &ws, Cursor &c) {
 // of the class per bucket and knows the lanes' keys; the next bucket's are loaded during the search.
 // One loop for all of them takes 5.83 against 5.51 ms at 10^8 u64 keys (lambda 7), 2.46 against
 // 2.29 ms at 5*10^7 (lambda 6).
-template <int S, bool SMALL = true>
+template <int S, bool SMALL = true, bool DENSE = false, bool MEET = false>
 __device__ __forceinline__ uint32_t search_class(const WarpSmem &ws, const uint2 *so, const ScanRange &sr, FastMod fm,
                                                  uint32_t k_lim, uint32_t searched, int lane, Cursor &c, uint32_t *pil,
                                                  size_t pstride) {
@@ -682,7 +718,7 @@ __device__ __forceinline__ uint32_t search_class(const WarpSmem &ws, const uint2
             c.L = so[(c.sc & 0xFFFFu) + i];
         }
         uint32_t pilot = 0;
-        const uint32_t code = place_batched<S, SMALL>(ws, L, s, sr, fm, k_lim, lane, &pilot);
+        const uint32_t code = place_batched<S, SMALL, DENSE, MEET>(ws, L, s, sr, fm, k_lim, lane, &pilot);
         if (code != PHOBIC_OK) return code;
         if (lane == 0) pil[(size_t)b * pstride] = pilot;
     }
@@ -690,6 +726,7 @@ __device__ __forceinline__ uint32_t search_class(const WarpSmem &ws, const uint2
 }
 
 // One partition's pilots.
+template <bool DENSE>
 __device__ __forceinline__ uint32_t search_partition(const SearchArgs &a, uint32_t *w, const WarpSmem &ws,
                                                      const SetDesc &d, uint32_t g, uint32_t p, int lane) {
     const uint32_t nonempty = a.part_state[g];
@@ -719,10 +756,24 @@ __device__ __forceinline__ uint32_t search_partition(const SearchArgs &a, uint32
         const uint32_t s = c.s, b = c.sc >> 16, st = c.sc & 0xFFFFu;
         advance(ws, c);
         uint32_t pilot = 0;
-        code = place_large(ws, so + st, s, sr, fm, k_lim, lane, &pilot);
+        code = place_large<DENSE>(ws, so + st, s, sr, fm, k_lim, lane, &pilot);
         if (code == PHOBIC_OK && lane == 0 && PHB_CHECK(b < a.buckets)) pil[(size_t)b * pstride] = pilot;
     }
     if (c.j < searched) c.L = so[(c.sc & 0xFFFFu) + lane_key(c.s, lane)];
+    // A class whose buckets meet themselves on many counters, in this partition, is searched with MEET.
+    auto dense_class = [&](auto size) {
+        constexpr int S = decltype(size)::value;
+        if (code != PHOBIC_OK) return;
+        code = ps < crowded(S) ? search_class<S, true, true, true>(ws, so, sr, fm, k_lim, searched, lane, c, pil, pstride)
+                               : search_class<S, true, true>(ws, so, sr, fm, k_lim, searched, lane, c, pil, pstride);
+    };
+    if constexpr (DENSE) {
+        if (sr.rounds <= 3) {
+            dense_class(std::integral_constant<int, 32>{});
+            dense_class(std::integral_constant<int, 16>{});
+            dense_class(std::integral_constant<int, 8>{});
+        }
+    }
     if (code == PHOBIC_OK) code = search_class<32>(ws, so, sr, fm, k_lim, searched, lane, c, pil, pstride);
     if (code == PHOBIC_OK) code = search_class<16>(ws, so, sr, fm, k_lim, searched, lane, c, pil, pstride);
     if (sr.rounds <= 3) {
@@ -1115,6 +1166,7 @@ int search_warps_per_cta(uint32_t buckets, uint32_t cap) {
     return (int)(fit < (size_t)kSearchWarps ? fit : (size_t)kSearchWarps);
 }
 
+template <bool DENSE>
 __global__ void __launch_bounds__(kSearchWarps * 32, kSearchCtasPerSm) k_search(SearchArgs a) {
     extern __shared__ __align__(16) uint32_t smem[];
     const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
@@ -1129,7 +1181,7 @@ __global__ void __launch_bounds__(kSearchWarps * 32, kSearchCtasPerSm) k_search(
         if (fatal_before_search(*reinterpret_cast<volatile unsigned long long *>(&a.err[s]))) continue;
         const SetDesc &d = a.sets[s];
         const uint32_t p = g - d.part_base;
-        const uint32_t code = search_partition(a, mine, ws, d, g, p, lane);
+        const uint32_t code = search_partition<DENSE>(a, mine, ws, d, g, p, lane);
         if (code != PHOBIC_OK && lane == 0) report_error(&a.err[s], p, code);
     }
 }
@@ -1188,15 +1240,16 @@ cudaError_t launch_search(const SearchArgs &a, int sm_count, cudaStream_t st, Se
     const int warps = search_warps_per_cta(a.buckets, a.cap);
     if (warps < 1) return cudaErrorInvalidValue;
     const size_t smem = (size_t)warps * search_warp_smem(a.buckets, a.cap);
-    cudaError_t e = allow_dynamic_smem(k_search, smem);
+    auto *kernel = a.partition_size <= kDenseSlots ? k_search<true> : k_search<false>;
+    cudaError_t e = allow_dynamic_smem(kernel, smem);
     if (e != cudaSuccess) return e;
     int per_sm = 0;
-    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_search, warps * 32, smem);
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kernel, warps * 32, smem);
     if (e != cudaSuccess) return e;
     if (per_sm < 1) per_sm = 1;
     uint64_t want = (a.M + warps - 1) / warps;
     int grid = (int)std::min<uint64_t>(want, (uint64_t)per_sm * sm_count);
-    k_search<<<grid, warps * 32, smem, st>>>(a);
+    kernel<<<grid, warps * 32, smem, st>>>(a);
     return cudaGetLastError();
 }
 
