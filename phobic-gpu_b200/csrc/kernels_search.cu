@@ -324,6 +324,9 @@ constexpr uint32_t kDenseSlots = 128;
 // about three quarters of S keys) that the test comes before the scan: search of 10^6 keys at P 32 77.8 ms
 // without, 49.1 with it, and 59.5 and 49.0 with limits of S * S and S * S / 4.
 constexpr uint32_t crowded(uint32_t S) { return S * S / 2; }
+// The same for the group kernel, whose searches test for it beside their scan: search of 30,000 strings at
+// P 64 2.52 ms without, 1.95 with it; the limits above make 10^5 keys at P 128 432 us instead of 399.
+constexpr uint32_t crowded_ahead(uint32_t S) { return 3 * S; }
 
 // Lanes per pilot counter for a bucket of s <= 32 keys: 4, 8, 16 or 32.
 __device__ __forceinline__ uint32_t counter_lanes(uint32_t s) { return s <= 4 ? 4u : s <= 8 ? 8u : s <= 16 ? 16u : 32u; }
@@ -455,6 +458,7 @@ template <int NR>
 struct Seek {
     uint32_t kb, k, o, h;
     uint32_t bad[NR ? NR : 1];
+    uint32_t mb, meet;  // crowded buckets: as `meet` in place_batched, of the batch that starts at mb
 };
 
 // The search of place_batched as the bucket pipeline runs it: nothing is marked, and it can be
@@ -480,6 +484,22 @@ __device__ __forceinline__ uint32_t seek_batched(const WarpSmem &ws, uint32_t *h
             hs[lane] = hk;
         }
         __syncwarp();
+        // A bucket that meets itself on most counters: what a failing one takes counts.
+        if (NR == 1 && S > 4 && sr.ps < crowded_ahead(S)) {
+            if (f->mb != f->k - u) {
+                f->mb = f->k - u;
+                const uint32_t same = same_slot_lanes<S>(hs[lane], s, lane);
+                f->meet = __ballot_sync(kFullMask, (same & (same - 1u)) != 0u);
+            }
+            if ((f->meet >> (S * u)) & (kFullMask >> (32 - S))) continue;
+            if constexpr (NR == 1) {
+                all_windows<S, NR>(ws, hs_sa + 4 * S * u, s, sr, lane, f->bad);
+                if (__all_sync(kFullMask, f->bad[0] == kFullMask)) continue;
+                f->o = smallest_offset<NR>(f->bad, lane);
+                f->h = unpack_slot(hs[S * u + (mine ? (uint32_t)lane : 0u)]);
+                return PHOBIC_OK;
+            }
+        }
         const uint32_t own = hs[S * u + (mine ? (uint32_t)lane : 0u)];
         bool meet = false;
         if constexpr (NR > 0) meet = all_windows<S, NR>(ws, hs_sa + 4 * S * u, s, sr, lane, f->bad);
@@ -987,6 +1007,7 @@ __device__ __forceinline__ void pipeline(const WarpSmem &ws, const uint2 *so, co
         read(j + 3 * W);
         Seek<NR> f;
         f.kb = f.k = f.o = f.h = 0;
+        f.mb = kNone;
         // One lane reads the status, which another warp may be writing: the warp agrees on what it saw.
         uint32_t st = __shfl_sync(kFullMask, lane == 0 ? *status : 0u, 0), q = 0, at = 0, bit = 0;
         bool turn = false, seek = st == PHOBIC_OK, on = false;
