@@ -439,6 +439,30 @@ __device__ __forceinline__ bool all_windows(const WarpSmem &ws, uint32_t hs, uin
     return false;
 }
 
+// Which of V counters have an open window, as bits: their buckets' packed slots, S = 4 or 8 of them each,
+// start at the shared address hs, in a partition of one round.  All loads of the V counters are in flight together.
+template <int S, int V>
+__device__ __forceinline__ uint32_t open_counters(const WarpSmem &ws, uint32_t hs, const ScanRange &sr, int lane) {
+    const uint32_t lane_sa = ws.occ + 8u * lane;
+    uint4 x[V * S / 4];
+#pragma unroll
+    for (int i = 0; i < V * S / 4; i++) x[i] = lds128(hs + 16 * i);
+    uint32_t bad[V];
+#pragma unroll
+    for (int v = 0; v < V; v++) {
+        bad[v] = sr.last_dead;
+#pragma unroll
+        for (int i = v * S / 4; i < (v + 1) * S / 4; i++) {
+            bad[v] |= window_at<0>(ws, lane_sa + (x[i].x >> 5), x[i].x) | window_at<0>(ws, lane_sa + (x[i].y >> 5), x[i].y);
+            bad[v] |= window_at<0>(ws, lane_sa + (x[i].z >> 5), x[i].z) | window_at<0>(ws, lane_sa + (x[i].w >> 5), x[i].w);
+        }
+    }
+    uint32_t open = 0;
+#pragma unroll
+    for (int v = 0; v < V; v++) open |= __any_sync(kFullMask, bad[v] != kFullMask) ? 1u << v : 0u;
+    return open;
+}
+
 // The warp's smallest free offset in these windows (kNone: none).
 template <int NR>
 __device__ __forceinline__ uint32_t smallest_offset(const uint32_t (&bad)[NR], int lane) {
@@ -472,6 +496,7 @@ __device__ __forceinline__ uint32_t seek_batched(const WarpSmem &ws, uint32_t *h
     constexpr uint32_t G = 32 / S;
     const uint32_t hs_sa = (uint32_t)__cvta_generic_to_shared(hs);
     const bool mine = lane < (int)s;
+    const uint32_t from = f->k;
 #pragma unroll 1
     for (;; ++f->k) {
         if (f->k >= k_lim) return PHOBIC_ERR_SEARCH_LIMIT;
@@ -498,6 +523,18 @@ __device__ __forceinline__ uint32_t seek_batched(const WarpSmem &ws, uint32_t *h
                 f->o = smallest_offset<NR>(f->bad, lane);
                 f->h = unpack_slot(hs[S * u + (mine ? (uint32_t)lane : 0u)]);
                 return PHOBIC_OK;
+            }
+        }
+        // One counter has failed: the next ones are looked at V at a time, up to the first with an open window
+        // (a partition of one round; V divides the batch, and counters past k_lim end the search above).
+        if constexpr (NR == 1 && S <= 8) {
+            constexpr uint32_t V = 16 / S;
+            if (f->k != from && u % V == 0) {
+                const uint32_t open = open_counters<S, V>(ws, hs_sa + 4 * S * u, sr, lane);
+                if (!(open & 1u)) {
+                    f->k += open ? __ffs(open) - 2 : V - 1;
+                    continue;
+                }
             }
         }
         const uint32_t own = hs[S * u + (mine ? (uint32_t)lane : 0u)];

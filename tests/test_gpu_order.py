@@ -92,7 +92,7 @@ def test_small_builds_report_errors_like_the_oracle(phobic):
 
 
 @pytest.mark.parametrize("group,pipe", [(1, 0), (4, 0), (2, 1), (4, 1), (8, 1), (0, 0)])
-@pytest.mark.parametrize("P,n", [(16, 20), (32, 200), (64, 9_000), (128, 30_000), (256, 1_000), (300, 40_000), (512, 90_000)])
+@pytest.mark.parametrize("P,n", [(16, 20), (32, 200), (64, 9_000), (128, 30_000), (256, 1_000), (300, 40_000), (512, 90_000), (520, 30_000)])
 def test_small_partitions_match_oracle(phobic, P, n, group, pipe):
     """Partitions of few slots: most offsets of a bucket's windows are gone by its turn, most of its
     pilot counters put two keys on one slot, and a partition is ordered by one warp."""
