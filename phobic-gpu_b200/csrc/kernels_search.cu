@@ -317,16 +317,18 @@ __device__ __forceinline__ bool slots_distinct(uint32_t *scr, uint32_t q, bool o
 }
 
 // Builds of at most this many keys per partition are searched by the DENSE kernel: their partitions
-// need many counters, so what a failing one takes counts.  Search of 2*10^7 keys at P 128 19.9 ms without
-// it, 12.8 with it; at P 256 3.2 and 3.7.
+// need many counters, so what a failing one takes counts.  Search of 2*10^7 keys (lambda 5) at P 128 19.9 ms
+// without it, 10.9 with it; at P 256 2.05 and 2.25.
 constexpr uint32_t kDenseSlots = 128;
 // Slots below which a bucket of S / 2 to S keys meets itself on so many pilot counters (half of them, at
-// about three quarters of S keys) that the test comes before the scan: search of 10^6 keys at P 32 77.8 ms
-// without, 49.1 with it, and 59.5 and 49.0 with limits of S * S and S * S / 4.
+// about three quarters of S keys) that the test comes before the scan: search of 10^6 keys at P 32 77.9 ms
+// without, 46.2 with it; limits of twice and half as many slots make 43.8 and 46.2 of it, and 2.42 and 2.34
+// of 2.50 ms at 3*10^7 (P 128, lambda 3).
 constexpr uint32_t crowded(uint32_t S) { return S * S / 2; }
 // The same for the group kernel, whose searches test for it beside their scan: search of 30,000 strings at
-// P 64 2.52 ms without, 1.95 with it; the limits above make 10^5 keys at P 128 432 us instead of 399.
-constexpr uint32_t crowded_ahead(uint32_t S) { return 3 * S; }
+// P 64 2.52 ms without, 1.63 with it.  3 S slots for S = 16 and 32 make 176 us of 119 at 3*10^5 keys (P 128,
+// lambda 3), 5 S for S = 8, whose counters are also looked at two at a time, 323 of 237 at 1000 (P 32).
+constexpr uint32_t crowded_ahead(uint32_t S) { return S == 8 ? 3 * S : 5 * S; }
 
 // Lanes per pilot counter for a bucket of s <= 32 keys: 4, 8, 16 or 32.
 __device__ __forceinline__ uint32_t counter_lanes(uint32_t s) { return s <= 4 ? 4u : s <= 8 ? 8u : s <= 16 ? 16u : 32u; }
@@ -337,13 +339,17 @@ __device__ __forceinline__ uint32_t lane_key(uint32_t s, int lane) {
     return i < s ? i : 0u;
 }
 
-// The lanes whose packed slot is this lane's, among the keys of a bucket of s <= S keys under the same
-// counter (lane t * S + i: key i, counter t).
+// Lanes whose packed slot is also that of another key of their bucket of s <= S keys under the same counter
+// (lane t * S + i: key i, counter t), as a vote in which each such pair shows once at least.  S / 2 rotations
+// cover all pairs and are in flight together; __match_any_sync takes 360 cycles.
 template <int S>
-__device__ __forceinline__ uint32_t same_slot_lanes(uint32_t hk, uint32_t s, int lane) {
-    // Packed slots have 20 bits; lanes past the bucket take values of their own.
+__device__ __forceinline__ uint32_t meeting_lanes(uint32_t hk, uint32_t s, int lane) {
     const bool key = ((uint32_t)lane & (S - 1u)) < s;
-    return __match_any_sync(kFullMask, key ? hk | ((uint32_t)lane / S) << 24 : 0x80000000u | (uint32_t)lane);
+    const uint32_t v = key ? hk : 0x80000000u | (uint32_t)lane;  // lanes past the bucket: values of their own
+    bool meet = false;
+#pragma unroll
+    for (int r = 1; r <= S / 2; r++) meet |= v == __shfl_sync(kFullMask, v, lane + r, S);
+    return __ballot_sync(kFullMask, meet);
 }
 
 // A bucket of at most S keys (S = 4, 8, 16 or 32; more than S / 2 of them, or S = 4), L as
@@ -369,9 +375,8 @@ __device__ __forceinline__ uint32_t place_batched(const WarpSmem &ws, uint2 L, u
         const uint32_t hk = MEET ? hk_next : pack_slot(fm.mod(pilot_hash(L.x, L.y, k0 + (uint32_t)lane / S)));
         uint32_t meet = 0;  // lanes whose slot is that of another key under their counter
         if constexpr (MEET) {
-            const uint32_t same = same_slot_lanes<S>(hk, s, lane);
-            hk_next = pack_slot(fm.mod(pilot_hash(L.x, L.y, k0 + G + (uint32_t)lane / S)));  // during the match
-            meet = __ballot_sync(kFullMask, (same & (same - 1u)) != 0u);
+            hk_next = pack_slot(fm.mod(pilot_hash(L.x, L.y, k0 + G + (uint32_t)lane / S)));
+            meet = meeting_lanes<S>(hk, s, lane);
             if (G == 1 && meet) continue;
         }
         __syncwarp();
@@ -482,7 +487,7 @@ template <int NR>
 struct Seek {
     uint32_t kb, k, o, h;
     uint32_t bad[NR ? NR : 1];
-    uint32_t mb, meet;  // crowded buckets: as `meet` in place_batched, of the batch that starts at mb
+    uint32_t tested, apart;  // seek_crowded: the batch that was tested for keys that meet, its counters without
 };
 
 // The search of place_batched as the bucket pipeline runs it: nothing is marked, and it can be
@@ -509,22 +514,6 @@ __device__ __forceinline__ uint32_t seek_batched(const WarpSmem &ws, uint32_t *h
             hs[lane] = hk;
         }
         __syncwarp();
-        // A bucket that meets itself on most counters: what a failing one takes counts.
-        if (NR == 1 && S > 4 && sr.ps < crowded_ahead(S)) {
-            if (f->mb != f->k - u) {
-                f->mb = f->k - u;
-                const uint32_t same = same_slot_lanes<S>(hs[lane], s, lane);
-                f->meet = __ballot_sync(kFullMask, (same & (same - 1u)) != 0u);
-            }
-            if ((f->meet >> (S * u)) & (kFullMask >> (32 - S))) continue;
-            if constexpr (NR == 1) {
-                all_windows<S, NR>(ws, hs_sa + 4 * S * u, s, sr, lane, f->bad);
-                if (__all_sync(kFullMask, f->bad[0] == kFullMask)) continue;
-                f->o = smallest_offset<NR>(f->bad, lane);
-                f->h = unpack_slot(hs[S * u + (mine ? (uint32_t)lane : 0u)]);
-                return PHOBIC_OK;
-            }
-        }
         // One counter has failed: the next ones are looked at V at a time, up to the first with an open window
         // (a partition of one round; V divides the batch, and counters past k_lim end the search above).
         if constexpr (NR == 1 && S <= 8) {
@@ -558,9 +547,56 @@ __device__ __forceinline__ uint32_t seek_batched(const WarpSmem &ws, uint32_t *h
         if (!meet && f->o != kNone) return PHOBIC_OK;
     }
 }
+// seek_batched for a bucket that meets itself on most counters, in a partition of one round: the counters
+// of a batch that do are found at once and passed over.
+template <int S>
+__device__ __forceinline__ uint32_t seek_crowded(const WarpSmem &ws, uint32_t *hs, uint2 L, uint32_t s,
+                                                 const ScanRange &sr, FastMod fm, uint32_t k_lim, int lane, Seek<1> *f) {
+    constexpr uint32_t G = 32 / S;
+    const uint32_t hs_sa = (uint32_t)__cvta_generic_to_shared(hs);
+#pragma unroll 1
+    for (;; ++f->k) {
+        if (f->k >= k_lim) return PHOBIC_ERR_SEARCH_LIMIT;
+        uint32_t u = f->k % G;
+        if (f->k - u != f->kb) {  // u = 0
+            if (f->k == kDupCheckAt && s > 1 && has_duplicate_key(L, s, lane)) return PHOBIC_ERR_DUPLICATE_KEY;
+            f->kb = f->k;
+            const uint32_t hk = pack_slot(fm.mod(pilot_hash(L.x, L.y, f->k + (uint32_t)lane / S)));
+            __syncwarp();
+            hs[lane] = hk;
+        }
+        __syncwarp();
+        if (f->tested != f->kb) {
+            f->tested = f->kb;
+            const uint32_t meet = meeting_lanes<S>(hs[lane], s, lane);
+            f->apart = 0;
+#pragma unroll
+            for (uint32_t t = 0; t < G; t++) f->apart |= (meet >> (S * t)) & (kFullMask >> (32 - S)) ? 0u : 1u << t;
+        }
+        const uint32_t next = f->apart >> u;
+        const uint32_t skip = next ? __ffs(next) - 1 : G - u;
+        f->k += skip;
+        u += skip;
+        if (u == G) {
+            --f->k;
+            continue;
+        }
+        if (f->k >= k_lim) return PHOBIC_ERR_SEARCH_LIMIT;
+        all_windows<S, 1>(ws, hs_sa + 4 * S * u, s, sr, lane, f->bad);
+        if (__all_sync(kFullMask, f->bad[0] == kFullMask)) continue;
+        f->o = smallest_offset<1>(f->bad, lane);
+        f->h = unpack_slot(hs[S * u + (lane < (int)s ? (uint32_t)lane : 0u)]);
+        return PHOBIC_OK;
+    }
+}
 template <int NR>
 __device__ __forceinline__ uint32_t seek_any(const WarpSmem &ws, uint32_t *hs, uint2 L, uint32_t s, const ScanRange &sr,
                                              FastMod fm, uint32_t k_lim, int lane, Seek<NR> *f) {
+    if constexpr (NR == 1) {
+        if (s > 16 && sr.ps < crowded_ahead(32)) return seek_crowded<32>(ws, hs, L, s, sr, fm, k_lim, lane, f);
+        if (s > 8 && s <= 16 && sr.ps < crowded_ahead(16)) return seek_crowded<16>(ws, hs, L, s, sr, fm, k_lim, lane, f);
+        if (s > 4 && s <= 8 && sr.ps < crowded_ahead(8)) return seek_crowded<8>(ws, hs, L, s, sr, fm, k_lim, lane, f);
+    }
     if (s <= 4) return seek_batched<4, NR>(ws, hs, L, s, sr, fm, k_lim, lane, f);
     if (s <= 8) return seek_batched<8, NR>(ws, hs, L, s, sr, fm, k_lim, lane, f);
     if (s <= 16) return seek_batched<16, NR>(ws, hs, L, s, sr, fm, k_lim, lane, f);
@@ -1044,7 +1080,7 @@ __device__ __forceinline__ void pipeline(const WarpSmem &ws, const uint2 *so, co
         read(j + 3 * W);
         Seek<NR> f;
         f.kb = f.k = f.o = f.h = 0;
-        f.mb = kNone;
+        f.tested = kNone;
         // One lane reads the status, which another warp may be writing: the warp agrees on what it saw.
         uint32_t st = __shfl_sync(kFullMask, lane == 0 ? *status : 0u, 0), q = 0, at = 0, bit = 0;
         bool turn = false, seek = st == PHOBIC_OK, on = false;
