@@ -207,6 +207,45 @@ __device__ __forceinline__ bool order_parallel(const SearchArgs &a, uint32_t g, 
     return true;
 }
 
+// Looks a partition up, by one thread, so that those who order it agree on what becomes of it:
+// {base, size, state, -, pilots, partitions}.
+__device__ __forceinline__ void look_up(const SearchArgs &a, uint32_t g, uint32_t *in) {
+    const uint32_t s_idx = a.nsets == 1 ? 0u : find_set(a.part_base, a.nsets, g);
+    const SetDesc &d = a.sets[s_idx];
+    const uint32_t p = g - d.part_base;
+    const uint32_t base = a.G[g], end = a.G[g + 1];
+    const uint32_t ps = end - base;
+    // The size check comes first and looks at every partition, also of a set that failed before
+    // (only a scan that timed out leaves no offsets to check): the error word then holds the
+    // lowest oversized partition, whichever CTA comes to its own first.
+    const unsigned long long e = *reinterpret_cast<volatile unsigned long long *>(&a.err[s_idx]);
+    uint32_t state = 0;
+    if (e != kNoError && (uint32_t)e == PHOBIC_ERR_TIMEOUT) {
+        state = kPartSkipped;
+    } else if (ps > a.cap) {
+        report_error(&a.err[s_idx], p, PHOBIC_ERR_PARTITION_OVERFLOW);
+        state = kPartSkipped;
+    } else if (fatal_before_search(e)) {
+        state = kPartSkipped;
+    } else {
+        if (d.part_off) {
+            const uint32_t g0 = a.G[d.part_base];
+            d.part_off[p] = base - g0;
+            if (p + 1 == d.partitions) d.part_off[p + 1] = end - g0;
+        }
+        if (!PHB_CHECK(base + ps <= a.G[a.M])) {
+            state = kPartSkipped;
+        } else if (a.part_state[g] != end) {
+            // K3 placed exactly the keys K1 counted, unless the keys changed in between.
+            state = kPartSkipped | PHOBIC_ERR_KEYS_CHANGED;
+        }
+    }
+    if (state) a.part_state[g] = state;
+    const unsigned long long pil = reinterpret_cast<unsigned long long>(d.pilots + p);
+    in[0] = base, in[1] = ps, in[2] = state, in[4] = (uint32_t)pil, in[5] = (uint32_t)(pil >> 32);
+    in[6] = d.partitions;
+}
+
 }  // namespace
 
 __global__ void __launch_bounds__(kOrderThreads, kOrderCtas) k_order(SearchArgs a, uint32_t stage_keys) {
@@ -220,46 +259,8 @@ __global__ void __launch_bounds__(kOrderThreads, kOrderCtas) k_order(SearchArgs 
     uint32_t *info = sched + B + 1;  // {base, size, state, nonempty, pilots, partitions} by parity
     const bool parallel = B <= kOrderParallel;
 
-    // One thread looks a partition up, so that the CTA agrees on what becomes of it.
-    auto look_up = [&](uint32_t g, uint32_t *in) {
-        const uint32_t s_idx = a.nsets == 1 ? 0u : find_set(a.part_base, a.nsets, g);
-        const SetDesc &d = a.sets[s_idx];
-        const uint32_t p = g - d.part_base;
-        const uint32_t base = a.G[g], end = a.G[g + 1];
-        const uint32_t ps = end - base;
-        // The size check comes first and looks at every partition, also of a set that failed before
-        // (only a scan that timed out leaves no offsets to check): the error word then holds the
-        // lowest oversized partition, whichever CTA comes to its own first.
-        const unsigned long long e = *reinterpret_cast<volatile unsigned long long *>(&a.err[s_idx]);
-        uint32_t state = 0;
-        if (e != kNoError && (uint32_t)e == PHOBIC_ERR_TIMEOUT) {
-            state = kPartSkipped;
-        } else if (ps > a.cap) {
-            report_error(&a.err[s_idx], p, PHOBIC_ERR_PARTITION_OVERFLOW);
-            state = kPartSkipped;
-        } else if (fatal_before_search(e)) {
-            state = kPartSkipped;
-        } else {
-            if (d.part_off) {
-                const uint32_t g0 = a.G[d.part_base];
-                d.part_off[p] = base - g0;
-                if (p + 1 == d.partitions) d.part_off[p + 1] = end - g0;
-            }
-            if (!PHB_CHECK(base + ps <= a.G[a.M])) {
-                state = kPartSkipped;
-            } else if (a.part_state[g] != end) {
-                // K3 placed exactly the keys K1 counted, unless the keys changed in between.
-                state = kPartSkipped | PHOBIC_ERR_KEYS_CHANGED;
-            }
-        }
-        if (state) a.part_state[g] = state;
-        const unsigned long long pil = reinterpret_cast<unsigned long long>(d.pilots + p);
-        in[0] = base, in[1] = ps, in[2] = state, in[4] = (uint32_t)pil, in[5] = (uint32_t)(pil >> 32);
-        in[6] = d.partitions;
-    };
-
     uint32_t par = 0;
-    if (tid == 0 && blockIdx.x < a.M) look_up(blockIdx.x, info);
+    if (tid == 0 && blockIdx.x < a.M) look_up(a, blockIdx.x, info);
     for (uint32_t g = blockIdx.x; g < a.M; g += gridDim.x, par ^= kInfoWords) {
         for (uint32_t i = tid; i < B; i += kOrderThreads) cnt[i] = 0;
         for (uint32_t i = tid; i < table_words(B); i += kOrderThreads) tables[i] = 0;
@@ -287,7 +288,7 @@ __global__ void __launch_bounds__(kOrderThreads, kOrderCtas) k_order(SearchArgs 
             }
         }
         // The next partition is looked up meanwhile.
-        if (tid == kOrderThreads - 1 && g + gridDim.x < a.M) look_up(g + gridDim.x, info + (par ^ kInfoWords));
+        if (tid == kOrderThreads - 1 && g + gridDim.x < a.M) look_up(a, g + gridDim.x, info + (par ^ kInfoWords));
         if (state) continue;
 
         // Bucket sizes (bucket_sizes.comp:21-35).  Ids >= B never come from K3 for keys that K1
@@ -378,6 +379,129 @@ __global__ void __launch_bounds__(kOrderThreads, kOrderCtas) k_order(SearchArgs 
             if (ps && PHB_CHECK(i < 2 * ps)) sch[i] = sched[i];
         if (tid == 0) a.part_state[g] = nonempty;
     }
+}
+
+// ------------------------------------------------------------------ small partitions
+//
+// The same for partitions of few keys, one warp each: with so little to do in a partition, k_order's seven
+// barriers and its tables for 256 sizes are what takes the time, with 4 partitions in flight per SM.  Keys and
+// bucket ids of a partition of at most 32 ITEMS keys are in registers, and leave in bucket order through
+// shared memory.  3*10^7 keys: at P 64 0.96 ms of bucket order and partition passes instead of 4.1, at P 128
+// 0.78 instead of 2.3, at P 256 0.69 instead of 1.4, at P 512 0.62 instead of 0.92; larger partitions would
+// not fit the registers.
+constexpr int kWarpOrderThreads = 128;
+constexpr uint32_t kWarpOrderKeys = 512, kWarpOrderBuckets = 512;
+__host__ __device__ __forceinline__ size_t warp_order_words(uint32_t B, uint32_t stage_keys) {
+    return (2 * (size_t)stage_keys + 256 + 2 * (size_t)B + 1 + 2 * kInfoWords + 1) & ~size_t(1);
+}
+
+template <int ITEMS>
+__global__ void __launch_bounds__(kWarpOrderThreads) k_order_warp(SearchArgs a) {
+    extern __shared__ __align__(16) uint32_t smem[];
+    constexpr uint32_t kStage = 32 * ITEMS;
+    const uint32_t B = a.buckets, lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const uint32_t warps = gridDim.x * (kWarpOrderThreads / 32);
+    uint2 *raw = reinterpret_cast<uint2 *>(smem + warp * warp_order_words(B, kStage));
+    uint32_t *tables = reinterpret_cast<uint32_t *>(raw + kStage);
+    uint32_t *cnt = tables + 256;
+    uint32_t *sched = cnt + B;
+    uint32_t *info = sched + B + 1;
+
+    uint32_t g = blockIdx.x * (kWarpOrderThreads / 32) + warp, par = 0;
+    if (lane == 0 && g < a.M) look_up(a, g, info);
+    for (; g < a.M; g += warps, par ^= kInfoWords) {
+        for (uint32_t i = lane; i < B; i += 32) cnt[i] = 0;
+        for (uint32_t i = lane; i < 256; i += 32) tables[i] = 0;
+        __syncwarp();
+        const uint32_t *in = info + par;
+        const uint32_t base = in[0], ps = in[1], state = in[2];
+        uint32_t *pil = reinterpret_cast<uint32_t *>((unsigned long long)in[4] | (unsigned long long)in[5] << 32);
+        const uint32_t pstride = in[6];
+        const bool staged = ps <= kStage;
+        const uint16_t *bk = a.bkt + base;
+        const uint2 *lo = a.lowers + base;
+        uint2 key[ITEMS];
+        uint32_t br[ITEMS];  // bucket, then bucket | rank << 16
+        if (!state && staged) {
+#pragma unroll
+            for (int j = 0; j < ITEMS; j++) {
+                const uint32_t i = 32 * j + lane;
+                br[j] = i < ps ? __ldcs(bk + i) : 0u;
+                key[j] = i < ps ? __ldcs(lo + i) : make_uint2(0, 0);
+            }
+        }
+        if (lane == 31 && g + warps < a.M) look_up(a, g + warps, info + (par ^ kInfoWords));
+        if (state) continue;
+
+        if (staged) {
+#pragma unroll
+            for (int j = 0; j < ITEMS; j++) {
+                if (32 * j + lane >= ps) continue;
+                const uint32_t b = min(br[j], B - 1);
+                (void)PHB_CHECK(b == br[j]);
+                br[j] = b | (atomicAdd(&cnt[b], 1u) << 16);
+            }
+        } else {
+            for (uint32_t i = lane; i < ps; i += 32) {
+                const uint32_t b = min((uint32_t)bk[i], B - 1);
+                if (PHB_CHECK(b == bk[i])) atomicAdd(&cnt[b], 1u);
+            }
+        }
+        __syncwarp();
+        bool over = false;
+        for (uint32_t b = lane; b < B; b += 32) {
+            const uint32_t s = cnt[b];
+            if (a.debug_sizes) a.debug_sizes[(size_t)g * B + b] = s;
+            if (s > kMaxBucket) over = true;
+            else if (s && PHB_CHECK(s <= kSizeBins)) half_add(tables, kSizeBins - s, 1);
+            else pil[(size_t)b * pstride] = 0;
+        }
+        if (__any_sync(kFullMask, over)) {
+            if (lane == 0) a.part_state[g] = kPartSkipped | PHOBIC_ERR_BUCKET_OVERFLOW;
+            continue;
+        }
+        __syncwarp();
+        const uint32_t nonempty = order_buckets(cnt, sched, tables, tables + 128, B, ps, (int)lane);
+        __syncwarp();
+
+        uint2 *so = a.sorted + base;
+        if (staged) {
+#pragma unroll
+            for (int j = 0; j < ITEMS; j++) {
+                if (32 * j + lane >= ps) continue;
+                const uint32_t pos = cnt[br[j] & 0xFFFFu] + (br[j] >> 16);
+                if (PHB_CHECK(pos < ps)) raw[pos] = key[j];
+            }
+            __syncwarp();
+            for (uint32_t i = lane; i < ps; i += 32) so[i] = raw[i];
+        } else {
+            for (uint32_t i = lane; i < ps; i += 32) {
+                const uint32_t pos = atomicAdd(&cnt[min((uint32_t)bk[i], B - 1)], 1u);
+                if (PHB_CHECK(pos < ps)) so[pos] = lo[i];
+            }
+            __syncwarp();
+        }
+        uint32_t *sch = reinterpret_cast<uint32_t *>(const_cast<uint2 *>(lo));
+        for (uint32_t i = lane; i <= nonempty; i += 32)
+            if (ps && PHB_CHECK(i < 2 * ps)) sch[i] = sched[i];
+        if (lane == 0) a.part_state[g] = nonempty;
+        __syncwarp();
+    }
+}
+
+template <int ITEMS>
+static cudaError_t launch_order_warp(const SearchArgs &a, int sm_count, cudaStream_t st) {
+    constexpr int warps = kWarpOrderThreads / 32;
+    const size_t smem = 4 * warps * warp_order_words(a.buckets, 32 * ITEMS);
+    cudaError_t e = allow_dynamic_smem(k_order_warp<ITEMS>, smem);
+    if (e != cudaSuccess) return e;
+    int per_sm = 0;
+    e = cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, k_order_warp<ITEMS>, kWarpOrderThreads, smem);
+    if (e != cudaSuccess) return e;
+    if (per_sm < 1) per_sm = 1;
+    const int grid = (int)std::min<uint64_t>((a.M + warps - 1) / warps, (uint64_t)per_sm * (sm_count > 0 ? sm_count : 148));
+    k_order_warp<ITEMS><<<grid, kWarpOrderThreads, smem, st>>>(a);
+    return cudaGetLastError();
 }
 
 // ------------------------------------------------------------------ small builds
@@ -587,6 +711,12 @@ cudaError_t launch_order(const SearchArgs &a, int sm_count, cudaStream_t st) {
     // deviations above P leave room for kOrderCtas CTAs per SM.
     const double slack = 8.0 * std::sqrt((double)a.partition_size);
     const uint64_t want = std::min<uint64_t>((uint64_t)a.partition_size + (uint64_t)slack, a.cap);
+    if (a.partition_size <= kWarpOrderKeys && a.buckets <= kWarpOrderBuckets) {
+        if (want <= 128) return launch_order_warp<4>(a, sm_count, st);
+        if (want <= 256) return launch_order_warp<8>(a, sm_count, st);
+        if (want <= 512) return launch_order_warp<16>(a, sm_count, st);
+        return launch_order_warp<24>(a, sm_count, st);
+    }
     uint32_t stage_keys = (uint32_t)std::min<uint64_t>((want + 1) & ~1ull, kOrderThreads * kOrderItems);
     if (4 * order_words(a.buckets, stage_keys) > kSearchSmemLimit) stage_keys = 0;
     const size_t smem = 4 * order_words(a.buckets, stage_keys);
