@@ -495,7 +495,7 @@ struct Seek {
 // allows; kb is the first counter of the batch whose slots hs holds (kNone: none yet), so a
 // second call with the same k tests that counter again without a hash.  NR = 0: any number of
 // rounds, one after the other.
-template <int S, int NR>
+template <int S, int NR, bool FEW>
 __device__ __forceinline__ uint32_t seek_batched(const WarpSmem &ws, uint32_t *hs, uint2 L, uint32_t s,
                                                  const ScanRange &sr, FastMod fm, uint32_t k_lim, int lane, Seek<NR> *f) {
     constexpr uint32_t G = 32 / S;
@@ -515,8 +515,8 @@ __device__ __forceinline__ uint32_t seek_batched(const WarpSmem &ws, uint32_t *h
         }
         __syncwarp();
         // One counter has failed: the next ones are looked at V at a time, up to the first with an open window
-        // (a partition of one round; V divides the batch, and counters past k_lim end the search above).
-        if constexpr (NR == 1 && S <= 8) {
+        // (V divides the batch, and counters past k_lim end the search above).
+        if constexpr (FEW && S <= 8) {
             constexpr uint32_t V = 16 / S;
             if (f->k != from && u % V == 0) {
                 const uint32_t open = open_counters<S, V>(ws, hs_sa + 4 * S * u, sr, lane);
@@ -547,7 +547,7 @@ __device__ __forceinline__ uint32_t seek_batched(const WarpSmem &ws, uint32_t *h
         if (!meet && f->o != kNone) return PHOBIC_OK;
     }
 }
-// seek_batched for a bucket that meets itself on most counters, in a partition of one round: the counters
+// seek_batched for a bucket that meets itself on most counters, in a partition of few slots: the counters
 // of a batch that do are found at once and passed over.
 template <int S>
 __device__ __forceinline__ uint32_t seek_crowded(const WarpSmem &ws, uint32_t *hs, uint2 L, uint32_t s,
@@ -589,18 +589,18 @@ __device__ __forceinline__ uint32_t seek_crowded(const WarpSmem &ws, uint32_t *h
         return PHOBIC_OK;
     }
 }
-template <int NR>
+template <int NR, bool FEW>
 __device__ __forceinline__ uint32_t seek_any(const WarpSmem &ws, uint32_t *hs, uint2 L, uint32_t s, const ScanRange &sr,
                                              FastMod fm, uint32_t k_lim, int lane, Seek<NR> *f) {
-    if constexpr (NR == 1) {
+    if constexpr (FEW) {
         if (s > 16 && sr.ps < crowded_ahead(32)) return seek_crowded<32>(ws, hs, L, s, sr, fm, k_lim, lane, f);
         if (s > 8 && s <= 16 && sr.ps < crowded_ahead(16)) return seek_crowded<16>(ws, hs, L, s, sr, fm, k_lim, lane, f);
         if (s > 4 && s <= 8 && sr.ps < crowded_ahead(8)) return seek_crowded<8>(ws, hs, L, s, sr, fm, k_lim, lane, f);
     }
-    if (s <= 4) return seek_batched<4, NR>(ws, hs, L, s, sr, fm, k_lim, lane, f);
-    if (s <= 8) return seek_batched<8, NR>(ws, hs, L, s, sr, fm, k_lim, lane, f);
-    if (s <= 16) return seek_batched<16, NR>(ws, hs, L, s, sr, fm, k_lim, lane, f);
-    return seek_batched<32, NR>(ws, hs, L, s, sr, fm, k_lim, lane, f);
+    if (s <= 4) return seek_batched<4, NR, FEW>(ws, hs, L, s, sr, fm, k_lim, lane, f);
+    if (s <= 8) return seek_batched<8, NR, FEW>(ws, hs, L, s, sr, fm, k_lim, lane, f);
+    if (s <= 16) return seek_batched<16, NR, FEW>(ws, hs, L, s, sr, fm, k_lim, lane, f);
+    return seek_batched<32, NR, FEW>(ws, hs, L, s, sr, fm, k_lim, lane, f);
 }
 
 // One bucket of more than 32 keys (a few per partition).  Each try hashes chunk by chunk and
@@ -1027,16 +1027,20 @@ __device__ __forceinline__ uint32_t ksplit_bucket(const WarpSmem &ws, const uint
     }
 }
 
-// Offsets of a bucket's windows that are taken on its turn before the windows are read again (one
+// Partitions of few slots (FEW) have a pipeline of their own: most of the windows that a search saw are stale
+// by its turn, and most counters fail.  The same code for all partitions makes the search of 1000 keys
+// in one partition 50.2 us instead of 47.5, of 2,000 79.5 instead of 77.9.
+constexpr uint32_t kFewSlots = 768;
+// FEW: offsets of a bucket's windows that are taken on its turn before the windows are read again (one
 // look at the slots and one reduction each; reading them anew takes about three times as long).  In
 // partitions of few slots nearly all offsets of the first buckets' windows are gone by their turn: with the windows
 // walked to their end the search of 1000 keys takes 189 us at P 256 and 177 at P 128, with 8, 4, 2 and 1
-// steps 52, 46, 40 and 36 at P 256; at P 2048, where steps are few, 1 and 2 are up to 4 % slower than 4.
+// steps 52, 46, 40 and 36 at P 256 (and up to 4 % more at P 2048, where steps are few, with 1 and 2).
 constexpr uint32_t kStaleSteps = 4;
 
 // The bucket pipeline of a group from bucket `first` on (see k_search_group); NR as in
 // seek_batched.
-template <int W, int NR>
+template <int W, int NR, bool FEW = false>
 __device__ __forceinline__ void pipeline(const WarpSmem &ws, const uint2 *so, const ScanRange &sr, FastMod fm,
                                          uint32_t k_lim, uint32_t first, uint32_t nonempty, int w, int lane,
                                          uint32_t turn_id, uint32_t next_id, volatile uint32_t *status,
@@ -1087,7 +1091,7 @@ __device__ __forceinline__ void pipeline(const WarpSmem &ws, const uint2 *so, co
         uint32_t gone = 0;
 #pragma unroll 1
         for (;;) {
-            if (seek) st = seek_any<NR>(ws, ws.hs + half, L, s, sr, fm, k_lim, lane, &f);
+            if (seek) st = seek_any<NR, FEW>(ws, ws.hs + half, L, s, sr, fm, k_lim, lane, &f);
             on = lane < (int)s && st == PHOBIC_OK && PHB_CHECK(f.h < sr.ps && f.o < sr.ps);
             q = f.h + f.o;
             q = q >= sr.ps ? q - sr.ps : q;
@@ -1103,7 +1107,7 @@ __device__ __forceinline__ void pipeline(const WarpSmem &ws, const uint2 *so, co
             // a few of them were gone too, of the windows as they are now, or the next counter.
             seek = true;
             if constexpr (NR > 0) {
-                if (++gone % kStaleSteps != 0) {
+                if (!FEW || ++gone % kStaleSteps != 0) {
 #pragma unroll
                     for (int r = 0; r < NR; r++)
                         if (f.o >> 5 == (uint32_t)(32 * r + lane)) f.bad[r] |= 1u << (f.o & 31);
@@ -1218,7 +1222,8 @@ __global__ void __launch_bounds__(kSearchWarps * 32, 2) k_search_group(SearchArg
             }
             if (PIPE && err == PHOBIC_OK && j < searched) {
                 volatile uint32_t *status = ctl + 2;
-                if (sr.rounds == 1) pipeline<W, 1>(ws, so, sr, fm, k_lim, j, searched, w, lane, turn_id, next_id, status, pil, pstride);
+                if (ps <= kFewSlots) pipeline<W, 1, true>(ws, so, sr, fm, k_lim, j, searched, w, lane, turn_id, next_id, status, pil, pstride);
+                else if (sr.rounds == 1) pipeline<W, 1>(ws, so, sr, fm, k_lim, j, searched, w, lane, turn_id, next_id, status, pil, pstride);
                 else if (sr.rounds == 2) pipeline<W, 2>(ws, so, sr, fm, k_lim, j, searched, w, lane, turn_id, next_id, status, pil, pstride);
                 else if (sr.rounds == 3) pipeline<W, 3>(ws, so, sr, fm, k_lim, j, searched, w, lane, turn_id, next_id, status, pil, pstride);
                 else pipeline<W, 0>(ws, so, sr, fm, k_lim, j, searched, w, lane, turn_id, next_id, status, pil, pstride);
