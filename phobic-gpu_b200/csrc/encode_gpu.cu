@@ -194,9 +194,10 @@ phobic_status run_encode_gpu(Worker &w, DeviceArena &out_arena, int pilot_encode
     PHB_TRY(w.pinned.reserve(4096), "pinned");
     cudaStream_t s = w.stream;
 
-    // Inputs on the device; the maxima and {size, keys}; the column table.
-    const size_t max_bytes = align256(8 + 4 * (size_t)cols);
-    const size_t need = align256(4 * npil) + align256(4 * noff) + max_bytes + align256(16) +
+    // Inputs on the device; {size, keys, largest offset code} and the columns' maxima, side by side; the
+    // column table.
+    const size_t info_bytes = align256(24), max_bytes = align256(4 * (size_t)cols);
+    const size_t need = align256(4 * npil) + align256(4 * noff) + info_bytes + max_bytes +
                         align256(sizeof(EncColumn) * (cols + 1)) + 4096;
     w.arena.reset();
     PHB_TRY(w.arena.reserve(need), "device arena");
@@ -208,11 +209,11 @@ phobic_status run_encode_gpu(Worker &w, DeviceArena &out_arena, int pilot_encode
         PHB_TRY(cudaMemcpyAsync(b, built->partition_offsets, 4 * noff, cudaMemcpyHostToDevice, s), "H2D offsets");
         d_pil = a, d_off = b;
     }
-    unsigned long long *d_cmax = static_cast<unsigned long long *>(w.arena.take(max_bytes));
-    uint32_t *d_max = reinterpret_cast<uint32_t *>(d_cmax + 1);
-    unsigned long long *d_info = static_cast<unsigned long long *>(w.arena.take(16));
+    unsigned long long *d_info = static_cast<unsigned long long *>(w.arena.take(info_bytes + max_bytes));
+    unsigned long long *d_cmax = d_info + 2;
+    uint32_t *d_max = reinterpret_cast<uint32_t *>(reinterpret_cast<char *>(d_info) + info_bytes);
     EncColumn *d_cols = static_cast<EncColumn *>(w.arena.take(sizeof(EncColumn) * (cols + 1)));
-    PHB_TRY(cudaMemsetAsync(d_cmax, 0, max_bytes, s), "memset");
+    PHB_TRY(cudaMemsetAsync(d_info, 0, info_bytes + max_bytes, s), "memset");
     const uint64_t per_col = mono ? npil : P;
     const uint32_t psize = params->partition_size;
     const int diff = offset_encoder == 0;

@@ -80,3 +80,20 @@ def test_gpu_encoding_rejects_other_encoders(phobic, ctx):
         with pytest.raises(phobic.PhobicError) as e:
             phobic.encode_gpu(ctx, built, cfg, pe, "diff")
         assert e.value.status == phobic.ERR_INVALID
+
+
+@pytest.mark.parametrize("pe", PILOT)
+def test_gpu_encoding_fits_its_memory_limit(phobic, ctx, pe):
+    """The device memory of a call: pilots, offsets, a word per column, one per call, the column table and
+    4 KB, in pieces of 256 bytes."""
+    cfg = phobic.MPHFconfig(8.0, 2048)
+    built = ctx.build(keygen.splitmix64(33, 50_000), cfg)
+    B, m = cfg.bucketCountPerPartition, built.partitions
+    assert B % 64 == 0
+    cols = B if pe == "interleaved_compact" else 1
+    limit = sum(-(-x // 256) * 256 for x in (4 * B * m, 4 * (m + 1), 4 * cols, 8, 32 * (cols + 1))) + 4096
+    want, _ = phobic.encode(built, cfg, pe, "diff")
+    with phobic.Context(0) as small:
+        small.set_memory_limit(limit)
+        got, _, _ = phobic.encode_gpu(small, built, cfg, pe, "diff")
+    assert got == want
