@@ -424,9 +424,10 @@ uint64_t sets_arena_bytes(const phobic_keys *sets, uint32_t nsets, const phobic_
 // ------------------------------------------------------------------ build
 
 // Largest build (in partitions) whose stages are replayed as a graph.  Measured on the B200
-// with device-resident keys and results (per build, graph against stage-by-stage launches):
-// 10^4 keys 0.387 against 0.396 ms, 10^6 keys (489 partitions) 0.4675 against 0.4745 ms, and
-// 10^7 keys (4,000 partitions) 1.933 against 1.917 ms, so large builds launch stage by stage.
+// with device-resident keys and results (per call, graph against stage-by-stage launches):
+// 10^4 keys 198 against 200 us, 10^5 keys 217 against 218, 10^6 keys (489 partitions) 460 against
+// 456, 4*10^6 keys (1,954 partitions) 620 against 616, 10^7 keys (4,000 partitions) 1,638 against
+// 1,571: a replay saves host time only, and large builds launch stage by stage.
 constexpr uint64_t kGraphMaxPartitions = 2048;
 
 phobic_status enqueue_sets(Worker &w, const phobic_keys *sets, uint32_t nsets, const phobic_params *params,

@@ -32,8 +32,12 @@
 // Buckets of at most 32 keys (nearly all of them) are hashed for 32 / S pilot
 // counters at once (S = 4, 8, 16 or 32 lanes per counter) into shared memory, from
 // where every lane reads the slots of one counter four at a time (broadcast 128-bit
-// loads).  Larger buckets read their keys from the bucket-ordered copy in global
-// memory.
+// loads).  Larger buckets keep their first 32 keys in registers and read the others from
+// the bucket-ordered copy in global memory.
+//
+// Two times in a comment are of two variants measured side by side when the choice was made,
+// in a kernel that was otherwise that of its day; the search of 10^8 u64 keys (lambda 7,
+// P 2500) now takes 4.96 ms.
 #include <algorithm>
 #include <type_traits>
 

@@ -124,3 +124,18 @@ def test_crowded_buckets_match_oracle(phobic):
                     continue
                 got = ctx.build(keys, cfg)
                 assert (got.pilots == want["pilots"]).all() and (got.partition_offsets == want["offsets"]).all()
+
+
+@pytest.mark.parametrize("group,pipe", [(1, 0), (4, 1), (8, 1), (2, 0)])
+def test_more_one_key_buckets_than_are_listed(phobic, group, pipe):
+    """Hundreds of buckets of one key per partition: the last 128 go by the list of free slots, those before them
+    by the search."""
+    cfg = phobic.MPHFconfig(1.5, 2048)
+    keys = keygen.splitmix64(8200, 30_000)
+    want = O.build(O.hash_keys(keys, "u64"), 2048, cfg.bucketCountPerPartition, cfg.getFulcs(), intermediates=True)
+    assert want["status"] == 0
+    assert (want["bucket_sizes"].reshape(-1, cfg.bucketCountPerPartition) == 1).sum(axis=1).min() > 128
+    with phobic.Context(0) as ctx:
+        ctx.set_tuning(search_group=group, search_pipeline=pipe)
+        got = ctx.build(keys, cfg)
+    assert (got.pilots == want["pilots"]).all() and (got.partition_offsets == want["offsets"]).all()
